@@ -966,6 +966,9 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
       return bail(e, "cudaMemcpy(state)");
   }
   c->scratch_n = (size_t)2 * ceil_div(2L * c->max_nh, 256) + (size_t)32 * c->max_L3 + 64;
+  // slice measurements: sums, output and the segments' partial sums
+  for (const ChainDev& d : c->ch)
+    c->scratch_n = std::max(c->scratch_n, (size_t)21 * d.L3 + 5 + slice_part_doubles(d.nxy, d.L3));
   if ((e = cudaMalloc(&c->scratch_d, sizeof(double) * c->scratch_n)) != cudaSuccess)
     return bail(e, "cudaMalloc(scratch)");
   if (c->max_L3 * 14 * sizeof(double) > 48 * 1024) {
@@ -979,13 +982,16 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
   return c;
 }
 
-int get_slices(lce_ctx* c, int chain, double*& out) {
+// scratch: slice sums [L3][14], the correlator kernel's output, the partial
+// sums of the slices' segments
+int get_slices(lce_ctx* c, int chain, int group, double*& out) {
   const ChainDev& ch = c->ch[chain];
   double* slices = c->scratch_d;
-  out = c->scratch_d + (size_t)14 * ch.L3;
-  if (c->prec == LCE_PREC_F64) launch_slice_sums<double>(c->ch_d + chain, ch.L3, slices, c->stream);
-  else launch_slice_sums<float>(c->ch_d + chain, ch.L3, slices, c->stream);
-  launch_correlators(slices, ch.L1, ch.L2, ch.L3, out, c->stream);
+  out = slices + (size_t)14 * ch.L3;
+  double* part = out + (size_t)7 * ch.L3 + 5;
+  if (c->prec == LCE_PREC_F64) launch_slice_sums<double>(c->ch_d + chain, group, ch.nxy, ch.L3, part, slices, c->stream);
+  else launch_slice_sums<float>(c->ch_d + chain, group, ch.nxy, ch.L3, part, slices, c->stream);
+  launch_correlators(slices, group, ch.L1, ch.L2, ch.L3, out, c->stream);
   CK(cudaGetLastError());
   return LCE_OK;
 }
@@ -1733,7 +1739,7 @@ int slab_fourier_fix(lce_slabs* S, int start, double step, double theta_switch, 
 // each slab's own device), gathered into the whole lattice's slices on slab
 // 0's device, and the correlators of lce_correlator formed there; h
 // receives the 7 L3 + 5 values of the correlator kernel's output
-int slab_slices(lce_slabs* S, std::vector<double>& h) {
+int slab_slices(lce_slabs* S, int group, std::vector<double>& h) {
   const int n = (int)S->slab.size(), nz = S->nz, L3 = S->L[2];
   lce_ctx* c0 = S->slab[0];
   double* slices = S->g_d + n;
@@ -1741,8 +1747,9 @@ int slab_slices(lce_slabs* S, std::vector<double>& h) {
   for (int k = 0; k < n; ++k) {
     lce_ctx* c = S->slab[k];
     DeviceScope ds_(c->device);
-    if (S->prec == LCE_PREC_F64) launch_slice_sums<double>(c->ch_d, nz + 2, c->scratch_d, c->stream);
-    else launch_slice_sums<float>(c->ch_d, nz + 2, c->scratch_d, c->stream);
+    double* part = c->scratch_d + (size_t)14 * (nz + 2);
+    if (S->prec == LCE_PREC_F64) launch_slice_sums<double>(c->ch_d, group, S->nxy, nz + 2, part, c->scratch_d, c->stream);
+    else launch_slice_sums<float>(c->ch_d, group, S->nxy, nz + 2, part, c->scratch_d, c->stream);
     SCK(cudaGetLastError());
     const size_t bytes = (size_t)14 * nz * sizeof(double);
     double* dst = slices + (size_t)14 * k * nz;
@@ -1754,7 +1761,7 @@ int slab_slices(lce_slabs* S, std::vector<double>& h) {
   }
   DeviceScope ds_(c0->device);
   for (int k = 1; k < n; ++k) SCK(cudaStreamWaitEvent(c0->stream, S->ev_sum[k], 0));
-  launch_correlators(slices, S->L[0], S->L[1], L3, out, c0->stream);
+  launch_correlators(slices, group, S->L[0], S->L[1], L3, out, c0->stream);
   SCK(cudaGetLastError());
   h.assign((size_t)7 * L3 + 5, 0.0);
   SCK(cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c0->stream));
@@ -2559,11 +2566,10 @@ int lce_gauge_functional(lce_ctx* c, int chain, double* value) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !value || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const ChainDev& ch = c->ch[chain];
-  const int nb = ceil_div(2L * ch.nh, 256);
   double* part = c->scratch_d;
-  double* out = c->scratch_d + nb;
-  if (c->prec == LCE_PREC_F64) launch_functional<double>(c->ch_d + chain, part, ch.nh, c->stream);
-  else launch_functional<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  const int nb = c->prec == LCE_PREC_F64 ? launch_functional<double>(c->ch_d + chain, part, ch.nh, c->stream)
+                                          : launch_functional<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  double* out = part + nb;
   launch_sum_partials(part, nb, 1, out, c->stream);
   CK(cudaGetLastError());
   double s;
@@ -2577,11 +2583,10 @@ int lce_theta(lce_ctx* c, int chain, double* theta) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !theta || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const ChainDev& ch = c->ch[chain];
-  const int nb = ceil_div(ch.nh, kBlock);
   double* part = c->scratch_d;
-  double* out = c->scratch_d + nb;
-  if (c->prec == LCE_PREC_F64) launch_gf_theta<double>(c->ch_d + chain, part, ch.nh, c->stream);
-  else launch_gf_theta<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  const int nb = c->prec == LCE_PREC_F64 ? launch_gf_theta<double>(c->ch_d + chain, part, ch.nh, c->stream)
+                                          : launch_gf_theta<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  double* out = part + nb;
   launch_sum_partials(part, nb, 1, out, c->stream);
   CK(cudaGetLastError());
   double s;
@@ -2596,7 +2601,7 @@ int lce_correlator(lce_ctx* c, int chain, double* corr_a, double* corr_u, double
   if (!c || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const int L3 = c->ch[chain].L3;
   double* out;
-  int rc = get_slices(c, chain, out);
+  int rc = get_slices(c, chain, kSliceFixed, out);
   if (rc) return rc;
   std::vector<double> h((size_t)7 * L3 + 5);
   CK(cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -2613,7 +2618,7 @@ int lce_polyakov(lce_ctx* c, int chain, double* slice, double* corr, double* mea
   if (!c || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const int L3 = c->ch[chain].L3;
   double* out;
-  int rc = get_slices(c, chain, out);
+  int rc = get_slices(c, chain, kSlicePolyakov, out);
   if (rc) return rc;
   std::vector<double> h((size_t)7 * L3 + 5);
   CK(cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -2629,7 +2634,7 @@ int lce_scalarcorr(lce_ctx* c, int chain, double* slice, double* corr, double* m
   if (!c || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const int L3 = c->ch[chain].L3;
   double* out;
-  int rc = get_slices(c, chain, out);
+  int rc = get_slices(c, chain, kSliceScalar, out);
   if (rc) return rc;
   std::vector<double> h((size_t)7 * L3 + 5);
   CK(cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -2644,11 +2649,10 @@ int lce_plaquette(lce_ctx* c, int chain, double* plaq) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !plaq || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
   const ChainDev& ch = c->ch[chain];
-  const int nb = ceil_div(2L * ch.nh, 256);
   double* part = c->scratch_d;
-  double* out = c->scratch_d + nb;
-  if (c->prec == LCE_PREC_F64) launch_plaquette<double>(c->ch_d + chain, part, ch.nh, c->stream);
-  else launch_plaquette<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  const int nb = c->prec == LCE_PREC_F64 ? launch_plaquette<double>(c->ch_d + chain, part, ch.nh, c->stream)
+                                          : launch_plaquette<float>(c->ch_d + chain, part, ch.nh, c->stream);
+  double* out = part + nb;
   launch_sum_partials(part, nb, 1, out, c->stream);
   CK(cudaGetLastError());
   double s;
@@ -3010,7 +3014,7 @@ int lce_slabs_correlator(lce_slabs* h, double* corr_a, double* corr_u, double* c
   lce_slabs* S = h;
   if (!S) return LCE_ERR_INVALID;
   std::vector<double> v;
-  if (int rc = slab_slices(S, v)) return rc;
+  if (int rc = slab_slices(S, kSliceFixed, v)) return rc;
   const int L3 = S->L[2];
   if (corr_a) std::memcpy(corr_a, v.data(), L3 * sizeof(double));
   if (corr_u) std::memcpy(corr_u, v.data() + L3, L3 * sizeof(double));
@@ -3023,7 +3027,7 @@ int lce_slabs_polyakov(lce_slabs* h, double* slice, double* corr, double* mean2)
   lce_slabs* S = h;
   if (!S) return LCE_ERR_INVALID;
   std::vector<double> v;
-  if (int rc = slab_slices(S, v)) return rc;
+  if (int rc = slab_slices(S, kSlicePolyakov, v)) return rc;
   const int L3 = S->L[2];
   if (slice) std::memcpy(slice, v.data() + 3 * L3, L3 * sizeof(double));
   if (corr) std::memcpy(corr, v.data() + 4 * L3, L3 * sizeof(double));
@@ -3035,7 +3039,7 @@ int lce_slabs_scalarcorr(lce_slabs* h, double* slice, double* corr, double* mean
   lce_slabs* S = h;
   if (!S) return LCE_ERR_INVALID;
   std::vector<double> v;
-  if (int rc = slab_slices(S, v)) return rc;
+  if (int rc = slab_slices(S, kSliceScalar, v)) return rc;
   const int L3 = S->L[2];
   if (slice) std::memcpy(slice, v.data() + 5 * L3, L3 * sizeof(double));
   if (corr) std::memcpy(corr, v.data() + 6 * L3, L3 * sizeof(double));

@@ -236,22 +236,22 @@ __global__ void __launch_bounds__(kBlock) it_half_kernel(const ChainDev* chp, co
 }
 
 // U_f(x,mu) = G(x) U(x,mu) G(x+mu)^+ and A_f(x) -> G(x) A(x) G(x)^+, one
-// thread per site of both parities
+// thread per site; the parities' tiles in turn (both_parities_site), so that
+// G is read from HBM once (256^3 FP32: 422 us, 5.4 TB/s; 447 us with one
+// parity after the other)
 template <typename R>
 __global__ void __launch_bounds__(kBlock) gauge_apply_kernel(const ChainDev* chp) {
   const ChainDev& ch = *chp;
-  const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= 2 * ch.nh) return;
-  const int eo = i >= ch.nh ? 1 : 0, oe = 1 - eo, s = i - eo * ch.nh, nh = ch.nh;
+  const int nh = ch.nh;
+  int eo, s;
+  if (!both_parities_site(blockIdx.x, nh, eo, s)) return;
+  const int oe = 1 - eo;
   const Coord X = site_coord(eo, s, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
+  const NbrOff o = nbr_offsets(ch, X);
   const su2<R> gx = LinkIO<R>::ld(ch.g, (size_t)eo * nh + s);
-  const int L[3] = {ch.L1, ch.L2, ch.L3};
 #pragma unroll
   for (int mu = 0; mu < 3; ++mu) {
-    int c[3] = {X.x, X.y, X.z};
-    c[mu] = wrap(c[mu] + 1, L[mu]);
-    const int sp = site_index(c[0], c[1], c[2], ch.hx, ch.nxy);
-    const su2<R> gp = LinkIO<R>::ld(ch.g, (size_t)oe * nh + sp);
+    const su2<R> gp = LinkIO<R>::ld(ch.g, (size_t)oe * nh + (s + o.p[mu]));
     const size_t li = ((size_t)(mu * 2 + eo)) * nh + s;
     LinkIO<R>::st(ch.uf, li, unitarise64(nd(nn(gx, LinkIO<R>::ld(ch.u, li)), gp)));
   }
@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(1024) gf_check_kernel(const ChainDev* chp, Cha
   pdl_wait();
   if (cst->gf_done) return;
   double v[1] = {0.0};
+#pragma unroll 8
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v[0] += part[b];
   __shared__ double tot;
   block_reduce_store<1>(v, &tot);
@@ -335,11 +336,14 @@ __global__ void __launch_bounds__(kBlock) gf_theta_kernel(const ChainDev* chp, d
   block_reduce_store<1>(th, part + blockIdx.x);
 }
 
+// One block; eight records in flight per thread before their in-order adds
+// (one at a time, 65,536 records took 28 us at 256^3)
 template <int NQ>
 __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* part, int nblocks, double* out) {
   double v[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+#pragma unroll 8
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] += part[(size_t)b * NQ + q];
@@ -380,7 +384,7 @@ void launch_it_iteration(const ChainDev* ch, ChainState* cst, int flags, int ren
 
 template <typename R>
 void launch_gauge_apply(const ChainDev* ch, int nh, cudaStream_t s) {
-  gauge_apply_kernel<R><<<ceil_div(2L * nh, kBlock), kBlock, 0, s>>>(ch);
+  gauge_apply_kernel<R><<<2 * ceil_div(nh, kBlock), kBlock, 0, s>>>(ch);
 }
 
 template <typename R>
@@ -394,8 +398,10 @@ template void launch_transform_identity<float>(void*, int, cudaStream_t);
 template void launch_transform_identity<double>(void*, int, cudaStream_t);
 
 template <typename R>
-void launch_gf_theta(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
-  gf_theta_kernel<R><<<ceil_div(nh, kBlock), kBlock, 0, s>>>(ch, part);
+int launch_gf_theta(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
+  const int nb = ceil_div(nh, kBlock);
+  gf_theta_kernel<R><<<nb, kBlock, 0, s>>>(ch, part);
+  return nb;
 }
 
 void launch_sum_partials(const double* part, int nblocks, int nq, double* out, cudaStream_t s) {
@@ -421,7 +427,7 @@ template int launch_it_half<double>(const ChainDev*, ChainState*, int, int, doub
 
 template void launch_it_iteration<float>(const ChainDev*, ChainState*, int, int, double*, int, cudaStream_t);
 template void launch_it_iteration<double>(const ChainDev*, ChainState*, int, int, double*, int, cudaStream_t);
-template void launch_gf_theta<float>(const ChainDev*, double*, int, cudaStream_t);
-template void launch_gf_theta<double>(const ChainDev*, double*, int, cudaStream_t);
+template int launch_gf_theta<float>(const ChainDev*, double*, int, cudaStream_t);
+template int launch_gf_theta<double>(const ChainDev*, double*, int, cudaStream_t);
 
 }  // namespace lce

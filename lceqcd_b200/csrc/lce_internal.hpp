@@ -62,6 +62,36 @@ struct ChainDev {
   void* g;   // gauge transform of the last tracked gauge fixing, [parity][site]
 };
 
+// Neighbour offsets of one site.  The half-row index s = z*nxy + y*hx + (x>>1)
+// of f/adresses.f is a sum of per-axis terms, so the index of any neighbour,
+// one step or two steps along different axes, is s plus the steps' offsets;
+// p[k] / m[k] are the offsets of +1 / -1 along axis k (periodic).  Computed
+// once per site instead of re-deriving every neighbour from coordinates.
+struct NbrOff {
+  int p[3], m[3];
+};
+__device__ __forceinline__ NbrOff nbr_offsets(const ChainDev& ch, Coord X) {
+  NbrOff o;
+  const int xh = X.x >> 1;
+  o.p[0] = X.x + 1 == ch.L1 ? -xh : ((X.x + 1) >> 1) - xh;
+  o.m[0] = X.x == 0 ? ch.hx - 1 : ((X.x - 1) >> 1) - xh;
+  o.p[1] = X.y + 1 == ch.L2 ? ch.hx - ch.nxy : ch.hx;
+  o.m[1] = X.y == 0 ? ch.nxy - ch.hx : -ch.hx;
+  o.p[2] = X.z + 1 == ch.L3 ? ch.nxy - ch.nh : ch.nxy;
+  o.m[2] = X.z == 0 ? ch.nh - ch.nxy : -ch.nxy;
+  return o;
+}
+
+// The kernels that visit both parities take the tiles of kBlock sites of the
+// two parities in turn (block b: tile b / 2 of parity b % 2), so that the
+// other parity's neighbours are still in L2 where a whole parity is not: at
+// 256^3 one parity's links are 402 MB.
+__device__ __forceinline__ bool both_parities_site(int b, int nh, int& eo, int& s) {
+  eo = b & 1;
+  s = (b >> 1) * kBlock + (int)threadIdx.x;
+  return s < nh;
+}
+
 // mutable state shared by the chains of one context
 struct CtxState {
   unsigned long long pass_ctr;    // Philox pass counter
@@ -320,17 +350,25 @@ void* fa_gstep_ptr(void* buf, size_t vcap);
 // since the last call (kernel, line length, shared memory), or ""
 std::string fa_take_error();
 template <typename R>
-void launch_gf_theta(const ChainDev* ch, double* part, int nh, cudaStream_t s);
+int launch_gf_theta(const ChainDev* ch, double* part, int nh, cudaStream_t s);  // returns the number of partials
 void launch_sum_partials(const double* part, int nblocks, int nq, double* out, cudaStream_t s);
 
 // ---- measurements (lce_meas.cu)
+// the slice quantities a measurement needs (lce_meas.cu): of U_f and A_f (the
+// correlators), cos 4|A| (the Polyakov loop), |A|^2 (the scalar correlator)
+enum SliceGroup : int { kSliceFixed = 0, kSlicePolyakov = 1, kSliceScalar = 2 };
+// a group's slice sums of a chain's L3 planes of nxy sites per parity into
+// slices [L3][14] (the group's columns); part: slice_part_doubles of scratch
 template <typename R>
-void launch_slice_sums(const ChainDev* ch, int L3, double* slices, cudaStream_t s);
-void launch_correlators(const double* slices, int L1, int L2, int L3, double* out, cudaStream_t s);
+void launch_slice_sums(const ChainDev* ch, int group, int nxy, int L3, double* part, double* slices, cudaStream_t s);
+size_t slice_part_doubles(int nxy, int L3);
+void launch_correlators(const double* slices, int group, int L1, int L2, int L3, double* out, cudaStream_t s);
+// per-block partial sums; the number of blocks is returned, at most kSumBlocks
+constexpr int kSumBlocks = 148 * 16;
 template <typename R>
-void launch_plaquette(const ChainDev* ch, double* part, int nh, cudaStream_t s);
+int launch_plaquette(const ChainDev* ch, double* part, int nh, cudaStream_t s);
 template <typename R>
-void launch_functional(const ChainDev* ch, double* part, int nh, cudaStream_t s);
+int launch_functional(const ChainDev* ch, double* part, int nh, cudaStream_t s);
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 

@@ -1,176 +1,262 @@
 // lce_meas.cu -- device reductions for the measurements.
 //
-// slice_sums_kernel: one block per z slice sums, over both parities and in
-// FP64, the quantities the reference accumulates per slice:
+// Slice quantities, summed per z slice over both parities in FP64 (the
+// reference accumulates them per slice):
 //   0..2   A_f                        f/correlator.f:58-59
 //   3..11  per mu: Im a, Im b, -Re b  of U_f  (Im a and -i b, :61-74)
 //   12     cos(4 |A|) on the un-fixed A     f/polyakov.f:52-55
 //   13     |A|^2 on the un-fixed A          f/scalarcorr.f:48-51
-// correlators_kernel then forms the periodic z autocorrelations of
-// f/correlator.f:139-164, f/polyakov.f:100-108 and f/scalarcorr.f:96-104
-// (all z = 0..L3-1, as the reference writes them) and the meas2a average.
+// A measurement sums only the quantities it reports (SliceGroup): the
+// correlators read U_f and A_f (60 bytes per FP32 site), the Polyakov loop
+// and the scalar correlator A alone (12 bytes).  slice_sums_kernel gives a
+// slice's sites to several blocks, slice_fold_kernel adds their partial sums
+// in segment order, and correlators_kernel forms the periodic z
+// autocorrelations of f/correlator.f:139-164, f/polyakov.f:100-108 and
+// f/scalarcorr.f:96-104 (all z = 0..L3-1, as the reference writes them) and
+// the meas2a average.
+#include <algorithm>
+
 #include "lce_internal.hpp"
 
 namespace lce {
 
 constexpr int kSliceQ = 14;
+constexpr int kSliceThreads = 256;
 
-template <typename R>
-__global__ void __launch_bounds__(256) slice_sums_kernel(const ChainDev* chp, double* slices) {
+// the quantities [q0, q0 + nq) of a group
+template <int GROUP>
+struct SliceCols {
+  static constexpr int q0 = GROUP == kSliceFixed ? 0 : (GROUP == kSlicePolyakov ? 12 : 13);
+  static constexpr int nq = GROUP == kSliceFixed ? 12 : 1;
+};
+
+// Sites of a slice one block sums: 1024 (4 per thread) up to 128 x 128
+// slices, so that 128^3 gives 2048 blocks and 64^3 256; 4096 for larger
+// slices, where there are blocks enough and the 12-quantity block reduction
+// (~200 warp instructions) is spread over more sites.  It depends on the
+// slice alone, so a z-slab adds a slice in the order of the whole lattice.
+__host__ __device__ constexpr int slice_seg_sites(int nxy) { return 2 * nxy <= 16384 ? 1024 : 4096; }
+int slice_segments(int nxy) { return ceil_div(2L * nxy, slice_seg_sites(nxy)); }
+
+// One block per (segment, slice).  Bound by HBM where the fields exceed L2;
+// the loads of four sites are in flight per thread.  At 256^3 in FP32 (ncu):
+// U_f and A_f 190 us (5.3 TB/s), cos 4|A| 53 us, |A|^2 36 us, against 706 us
+// for all quantities on every call with one block per slice, which left most
+// of the chip without work; at 128^3 33 / 12 / 9 against 175 us.
+template <typename R, int GROUP>
+__global__ void __launch_bounds__(kSliceThreads) slice_sums_kernel(const ChainDev* chp, double* part) {
   const ChainDev& ch = *chp;
-  const int z = blockIdx.x, nh = ch.nh, nxy = ch.nxy;
-  const R* Af = reinterpret_cast<const R*>(ch.af);
-  const R* A = reinterpret_cast<const R*>(ch.a);
-  double v[kSliceQ];
+  const int nh = ch.nh, nxy = ch.nxy, z = blockIdx.y;
+  constexpr int NQ = SliceCols<GROUP>::nq;
+  double v[NQ];
 #pragma unroll
-  for (int q = 0; q < kSliceQ; ++q) v[q] = 0.0;
-  for (int i = threadIdx.x; i < 2 * nxy; i += blockDim.x) {
+  for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+  const int seg = slice_seg_sites(nxy), i0 = blockIdx.x * seg, i1 = min(2 * nxy, i0 + seg);
+#pragma unroll 4
+  for (int i = i0 + (int)threadIdx.x; i < i1; i += kSliceThreads) {
     const int eo = i >= nxy ? 1 : 0;
     const int s = z * nxy + (i - eo * nxy);
+    const R* A = reinterpret_cast<const R*>(GROUP == kSliceFixed ? ch.af : ch.a) + (size_t)eo * 3 * nh + s;
+    const R a1 = __ldg(A), a2 = __ldg(A + nh), a3 = __ldg(A + 2 * (size_t)nh);
+    if constexpr (GROUP == kSliceFixed) {
+      v[0] += (double)a1;
+      v[1] += (double)a2;
+      v[2] += (double)a3;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) v[k] += (double)__ldg(Af + ((size_t)(eo * 3 + k)) * nh + s);
-#pragma unroll
-    for (int mu = 0; mu < 3; ++mu) {
-      su2<R> u = LinkIO<R>::ld(ch.uf, ((size_t)(mu * 2 + eo)) * nh + s);
-      v[3 + 3 * mu] += (double)u.a.im;
-      v[4 + 3 * mu] += (double)u.b.im;
-      v[5 + 3 * mu] += -(double)u.b.re;
+      for (int mu = 0; mu < 3; ++mu) {
+        const su2<R> u = LinkIO<R>::ld(ch.uf, ((size_t)(mu * 2 + eo)) * nh + s);
+        v[3 + 3 * mu] += (double)u.a.im;
+        v[4 + 3 * mu] += (double)u.b.im;
+        v[5 + 3 * mu] += -(double)u.b.re;
+      }
+    } else if constexpr (GROUP == kSlicePolyakov) {
+      const R r2 = a1 * a1 + a2 * a2 + a3 * a3;
+      v[0] += (double)cos((R)4 * sqrt(r2));
+    } else {
+      v[0] += (double)a1 * a1 + (double)a2 * a2 + (double)a3 * a3;
     }
-    const R a1 = __ldg(A + ((size_t)(eo * 3 + 0)) * nh + s), a2 = __ldg(A + ((size_t)(eo * 3 + 1)) * nh + s),
-            a3 = __ldg(A + ((size_t)(eo * 3 + 2)) * nh + s);
-    const R r2 = a1 * a1 + a2 * a2 + a3 * a3;
-    v[12] += (double)cos((R)4 * sqrt(r2));
-    v[13] += (double)a1 * a1 + (double)a2 * a2 + (double)a3 * a3;
   }
-  block_reduce_store<kSliceQ>(v, slices + (size_t)z * kSliceQ);
+  block_reduce_store<NQ>(v, part + ((size_t)z * gridDim.x + blockIdx.x) * NQ);
+}
+
+// slice z's quantities from its segments' partial sums: one warp per
+// quantity, lane l adds the segments l, l + 32, ... in order, then the tree
+__global__ void __launch_bounds__(kSliceThreads) slice_fold_kernel(const double* part, int nseg, int nq, int q0,
+                                                                   double* slices) {
+  pdl_wait();
+  const int z = blockIdx.x, lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < nq; q += kSliceThreads / 32) {
+    double v = 0.0;
+    for (int k = lane; k < nseg; k += 32) v += part[((size_t)z * nseg + k) * nq + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) slices[(size_t)z * kSliceQ + q0 + q] = v;
+  }
 }
 
 // out: corr_a[L3], corr_u[L3], corr_3[L3], pol_slice[L3], pol_corr[L3],
-//      sc_slice[L3], sc_corr[L3], af[3], pol_mean2, sc_mean
-__global__ void __launch_bounds__(256) correlators_kernel(const double* slices, int L1, int L2, int L3,
-                                                          double* out) {
-  extern __shared__ double sh[];  // [L3][kSliceQ], normalised by L1*L2
+//      sc_slice[L3], sc_corr[L3], af[3], pol_mean2, sc_mean; a group writes
+// its own parts.  One warp per displacement z (8 per block), its lanes over
+// the slices x0; every block holds all slice means in shared memory.
+constexpr int kCorrThreads = 256;
+template <int GROUP>
+__global__ void __launch_bounds__(kCorrThreads) correlators_kernel(const double* slices, int L1, int L2, int L3,
+                                                                   double* out) {
+  extern __shared__ double sh[];  // [nq][L3], normalised by L1*L2
+  constexpr int q0 = SliceCols<GROUP>::q0, NQ = SliceCols<GROUP>::nq;
   const double norm = 1.0 / ((double)L1 * (double)L2);
-  for (int i = threadIdx.x; i < L3 * kSliceQ; i += blockDim.x) sh[i] = slices[i] * norm;
-  __syncthreads();
-  double* corr_a = out;
-  double* corr_u = out + L3;
-  double* corr_3 = out + 2 * L3;
-  double* pol_slice = out + 3 * L3;
-  double* pol_corr = out + 4 * L3;
-  double* sc_slice = out + 5 * L3;
-  double* sc_corr = out + 6 * L3;
-  double* tail = out + 7 * L3;
-  for (int z = threadIdx.x; z < L3; z += blockDim.x) {
-    double ca = 0, cu = 0, c3 = 0, cp = 0, cs = 0;
-    for (int x0 = 0; x0 < L3; ++x0) {
-      const double* p = sh + x0 * kSliceQ;
-      const double* q = sh + ((x0 + z) % L3) * kSliceQ;
-      ca += p[0] * q[0] + p[1] * q[1] + p[2] * q[2];
-      // Re[s1 s1' + s2 conj(s2')], s1 = sum Im a (real), s2 = sum -i b
-      cu += p[3] * q[3] + (p[4] * q[4] + p[5] * q[5]);
-      cu += p[6] * q[6] + (p[7] * q[7] + p[8] * q[8]);
-      c3 += p[9] * q[9] + (p[10] * q[10] + p[11] * q[11]);
-      cp += p[12] * q[12];
-      cs += p[13] * q[13];
-    }
-    corr_a[z] = ca / L3;
-    corr_u[z] = cu / (L3 * 2.0);
-    corr_3[z] = c3 / L3;
-    pol_corr[z] = cp / L3;
-    sc_corr[z] = cs / L3;
-    pol_slice[z] = sh[z * kSliceQ + 12];
-    sc_slice[z] = sh[z * kSliceQ + 13];
+  pdl_wait();
+  for (int i = threadIdx.x; i < L3 * NQ; i += kCorrThreads) {
+    const int z = i / NQ, q = i - z * NQ;
+    sh[q * L3 + z] = slices[(size_t)z * kSliceQ + q0 + q] * norm;
   }
-  if (threadIdx.x == 0) {
-    double af0 = 0, af1 = 0, af2 = 0, ps = 0, ss = 0;
-    for (int z = 0; z < L3; ++z) {
-      af0 += sh[z * kSliceQ + 0];
-      af1 += sh[z * kSliceQ + 1];
-      af2 += sh[z * kSliceQ + 2];
-      ps += sh[z * kSliceQ + 12];
-      ss += sh[z * kSliceQ + 13];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z = blockIdx.x * (kCorrThreads / 32) + warp;
+  double* tail = out + 7 * L3;
+  constexpr int NC = GROUP == kSliceFixed ? 3 : 1;
+  if (z < L3) {
+    double c[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) c[k] = 0.0;
+    for (int x0 = lane; x0 < L3; x0 += 32) {
+      const int x1 = x0 + z < L3 ? x0 + z : x0 + z - L3;
+      auto pq = [&](int q) { return sh[q * L3 + x0] * sh[q * L3 + x1]; };
+      if constexpr (GROUP == kSliceFixed) {
+        c[0] += pq(0) + pq(1) + pq(2);
+        // Re[s1 s1' + s2 conj(s2')], s1 = sum Im a (real), s2 = sum -i b
+        c[1] += pq(3) + (pq(4) + pq(5));
+        c[1] += pq(6) + (pq(7) + pq(8));
+        c[2] += pq(9) + (pq(10) + pq(11));
+      } else {
+        c[0] += pq(0);
+      }
     }
-    tail[0] = af0 / L3;
-    tail[1] = af1 / L3;
-    tail[2] = af2 / L3;
-    tail[3] = (ps / L3) * (ps / L3);
-    tail[4] = ss / L3;
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) c[k] += __shfl_down_sync(0xffffffffu, c[k], o);
+    }
+    if (lane == 0) {
+      if constexpr (GROUP == kSliceFixed) {
+        out[z] = c[0] / L3;
+        out[L3 + z] = c[1] / (L3 * 2.0);
+        out[2 * L3 + z] = c[2] / L3;
+      } else {
+        double* d = out + (GROUP == kSlicePolyakov ? 3 : 5) * L3;
+        d[z] = sh[z];
+        d[L3 + z] = c[0] / L3;
+      }
+    }
+  }
+  // the averages over all slices
+  if (blockIdx.x == 0 && warp < (GROUP == kSliceFixed ? 3 : 1)) {
+    double m = 0.0;
+    for (int k = lane; k < L3; k += 32) m += sh[warp * L3 + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_down_sync(0xffffffffu, m, o);
+    if (lane == 0) {
+      if (GROUP == kSliceFixed) tail[warp] = m / L3;
+      else if (GROUP == kSlicePolyakov) tail[3] = (m / L3) * (m / L3);
+      else tail[4] = m / L3;
+    }
   }
 }
 
-// plaquette 1/2 Re Tr U_mu(x) U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+ over both parities
+// plaquette 1/2 Re Tr U_mu(x) U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+ over both
+// parities, each link read from HBM once (256^3 FP32: 199 us, 283 us with one
+// parity after the other).  A block sums several tiles, at most kSumBlocks
+// blocks in all, so that their partial sums are few.
 template <typename R>
-__global__ void __launch_bounds__(256) plaquette_kernel(const ChainDev* chp, double* part) {
+__global__ void __launch_bounds__(kBlock) plaquette_kernel(const ChainDev* chp, double* part) {
   const ChainDev& ch = *chp;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nh = ch.nh, ntiles = 2 * ((nh + kBlock - 1) / kBlock);
   double v[1] = {0.0};
-  if (i < 2 * ch.nh) {
-    const int eo = i >= ch.nh ? 1 : 0, oe = 1 - eo, s = i - eo * ch.nh;
+  for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
+    int eo, s;
+    if (!both_parities_site(b, nh, eo, s)) continue;
+    const int oe = 1 - eo;
     const Coord X = site_coord(eo, s, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
-    const int L[3] = {ch.L1, ch.L2, ch.L3};
-    int up[3];
+    const NbrOff o = nbr_offsets(ch, X);
+    su2<R> u[3], w[3][3];  // U_mu(x); w[mu][nu] = U_mu(x + nu), nu != mu
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
-      int c[3] = {X.x, X.y, X.z};
-      c[mu] = wrap(c[mu] + 1, L[mu]);
-      up[mu] = site_index(c[0], c[1], c[2], ch.hx, ch.nxy);
+      u[mu] = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + eo)) * nh + s);
+#pragma unroll
+      for (int nu = 0; nu < 3; ++nu)
+        if (nu != mu) w[mu][nu] = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + oe)) * nh + (s + o.p[nu]));
     }
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu)
 #pragma unroll
-      for (int nu = mu + 1; nu < 3; ++nu) {
-        su2<R> a = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + eo)) * ch.nh + s);
-        su2<R> b = LinkIO<R>::ld(ch.u, ((size_t)(nu * 2 + oe)) * ch.nh + up[mu]);
-        su2<R> d = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + oe)) * ch.nh + up[nu]);
-        su2<R> e = LinkIO<R>::ld(ch.u, ((size_t)(nu * 2 + eo)) * ch.nh + s);
-        v[0] += (double)nn(nn(a, b), dd(d, e)).a.re;
-      }
+      for (int nu = mu + 1; nu < 3; ++nu) v[0] += (double)nn(nn(u[mu], w[nu][mu]), dd(w[mu][nu], u[nu])).a.re;
   }
   block_reduce_store<1>(v, part + blockIdx.x);
 }
 
 // Landau functional: sum over links of U_f of c_mu Re a
 template <typename R>
-__global__ void __launch_bounds__(256) functional_kernel(const ChainDev* chp, double* part) {
+__global__ void __launch_bounds__(kBlock) functional_kernel(const ChainDev* chp, double* part) {
   const ChainDev& ch = *chp;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = 2 * ch.nh;
   double v[1] = {0.0};
-  if (i < 2 * ch.nh) {
+#pragma unroll 2
+  for (int i = blockIdx.x * kBlock + (int)threadIdx.x; i < n; i += gridDim.x * kBlock) {
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
       const double w = mu == 2 ? ch.alpha : 1.0;
-      su2<R> u = LinkIO<R>::ld(ch.uf, (size_t)mu * 2 * ch.nh + i);
+      su2<R> u = LinkIO<R>::ld(ch.uf, (size_t)mu * n + i);
       v[0] += w * (double)u.a.re;
     }
   }
   block_reduce_store<1>(v, part + blockIdx.x);
 }
 
-template <typename R>
-void launch_slice_sums(const ChainDev* ch, int L3, double* slices, cudaStream_t s) {
-  slice_sums_kernel<R><<<L3, 256, 0, s>>>(ch, slices);
+template <typename R, int GROUP>
+void slice_group(const ChainDev* ch, int nxy, int L3, double* part, double* slices, cudaStream_t s) {
+  const int nseg = slice_segments(nxy);
+  slice_sums_kernel<R, GROUP><<<dim3(nseg, L3), kSliceThreads, 0, s>>>(ch, part);
+  (void)launch_pdl(slice_fold_kernel, L3, kSliceThreads, 0, s, (const double*)part, nseg, SliceCols<GROUP>::nq,
+                   SliceCols<GROUP>::q0, slices);
 }
-void launch_correlators(const double* slices, int L1, int L2, int L3, double* out, cudaStream_t s) {
-  const size_t smem = (size_t)L3 * kSliceQ * sizeof(double);
+template <typename R>
+void launch_slice_sums(const ChainDev* ch, int group, int nxy, int L3, double* part, double* slices, cudaStream_t s) {
+  if (group == kSliceFixed) slice_group<R, kSliceFixed>(ch, nxy, L3, part, slices, s);
+  else if (group == kSlicePolyakov) slice_group<R, kSlicePolyakov>(ch, nxy, L3, part, slices, s);
+  else slice_group<R, kSliceScalar>(ch, nxy, L3, part, slices, s);
+}
+size_t slice_part_doubles(int nxy, int L3) { return (size_t)slice_segments(nxy) * L3 * SliceCols<kSliceFixed>::nq; }
+
+template <int GROUP>
+void corr_group(const double* slices, int L1, int L2, int L3, double* out, cudaStream_t s) {
+  const size_t smem = (size_t)L3 * SliceCols<GROUP>::nq * sizeof(double);
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(correlators_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  correlators_kernel<<<1, 256, smem, s>>>(slices, L1, L2, L3, out);
+    cudaFuncSetAttribute(correlators_kernel<GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  (void)launch_pdl(correlators_kernel<GROUP>, ceil_div(L3, kCorrThreads / 32), kCorrThreads, smem, s, slices, L1, L2,
+                   L3, out);
+}
+void launch_correlators(const double* slices, int group, int L1, int L2, int L3, double* out, cudaStream_t s) {
+  if (group == kSliceFixed) corr_group<kSliceFixed>(slices, L1, L2, L3, out, s);
+  else if (group == kSlicePolyakov) corr_group<kSlicePolyakov>(slices, L1, L2, L3, out, s);
+  else corr_group<kSliceScalar>(slices, L1, L2, L3, out, s);
 }
 template <typename R>
-void launch_plaquette(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
-  plaquette_kernel<R><<<ceil_div(2L * nh, 256), 256, 0, s>>>(ch, part);
+int launch_plaquette(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
+  const int nb = std::min(kSumBlocks, 2 * ceil_div(nh, kBlock));
+  plaquette_kernel<R><<<nb, kBlock, 0, s>>>(ch, part);
+  return nb;
 }
 template <typename R>
-void launch_functional(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
-  functional_kernel<R><<<ceil_div(2L * nh, 256), 256, 0, s>>>(ch, part);
+int launch_functional(const ChainDev* ch, double* part, int nh, cudaStream_t s) {
+  const int nb = std::min(kSumBlocks, ceil_div(2L * nh, kBlock));
+  functional_kernel<R><<<nb, kBlock, 0, s>>>(ch, part);
+  return nb;
 }
 
-template void launch_slice_sums<float>(const ChainDev*, int, double*, cudaStream_t);
-template void launch_slice_sums<double>(const ChainDev*, int, double*, cudaStream_t);
-template void launch_plaquette<float>(const ChainDev*, double*, int, cudaStream_t);
-template void launch_plaquette<double>(const ChainDev*, double*, int, cudaStream_t);
-template void launch_functional<float>(const ChainDev*, double*, int, cudaStream_t);
-template void launch_functional<double>(const ChainDev*, double*, int, cudaStream_t);
+template void launch_slice_sums<float>(const ChainDev*, int, int, int, double*, double*, cudaStream_t);
+template void launch_slice_sums<double>(const ChainDev*, int, int, int, double*, double*, cudaStream_t);
+template int launch_plaquette<float>(const ChainDev*, double*, int, cudaStream_t);
+template int launch_plaquette<double>(const ChainDev*, double*, int, cudaStream_t);
+template int launch_functional<float>(const ChainDev*, double*, int, cudaStream_t);
+template int launch_functional<double>(const ChainDev*, double*, int, cudaStream_t);
 
 }  // namespace lce

@@ -61,26 +61,6 @@ __device__ __forceinline__ R ldA(const R* A, int nh, int p, int k, int s) {
   return NC ? __ldg(q) : __ldcg(q);
 }
 
-// Neighbour offsets of one site.  The half-row index s = z*nxy + y*hx + (x>>1)
-// of f/adresses.f is a sum of per-axis terms, so the index of any neighbour,
-// one step or two steps along different axes, is s plus the steps' offsets;
-// p[k] / m[k] are the offsets of +1 / -1 along axis k (periodic).  Computed
-// once per site instead of re-deriving every neighbour from coordinates.
-struct NbrOff {
-  int p[3], m[3];
-};
-__device__ __forceinline__ NbrOff nbr_offsets(const ChainDev& ch, Coord X) {
-  NbrOff o;
-  const int xh = X.x >> 1;
-  o.p[0] = X.x + 1 == ch.L1 ? -xh : ((X.x + 1) >> 1) - xh;
-  o.m[0] = X.x == 0 ? ch.hx - 1 : ((X.x - 1) >> 1) - xh;
-  o.p[1] = X.y + 1 == ch.L2 ? ch.hx - ch.nxy : ch.hx;
-  o.m[1] = X.y == 0 ? ch.nxy - ch.hx : -ch.hx;
-  o.p[2] = X.z + 1 == ch.L3 ? ch.nxy - ch.nh : ch.nxy;
-  o.m[2] = X.z == 0 ? ch.nh - ch.nxy : -ch.nxy;
-  return o;
-}
-
 template <typename R, bool NC = true>
 __device__ __forceinline__ su2<R> ldU(const ChainDev& ch, int mu, int p, int s) {
   const size_t i = ((size_t)(mu * 2 + p)) * ch.nh + s;
