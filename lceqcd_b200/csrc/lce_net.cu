@@ -63,6 +63,14 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+// two floats rounded to a BF16 pair, and a pair's two values
+__device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return pack2(v.x, v.y);
+}
+__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
 // flat index of the neighbour at offset (dx, dy, dz) of flat site i
 __device__ __forceinline__ int nbr3(const NetGeom& g, int i, int dx, int dy, int dz) {
   const int eo = i >= g.nh ? 1 : 0, s = i - eo * g.nh;
@@ -158,16 +166,34 @@ __global__ void __launch_bounds__(32 * kConvWarps) conv_kernel(const __nv_bfloat
 // x-shifted sum with warp shuffles; the rows across warp boundaries go
 // through shared memory, and the two rows outside the tile (P_-1 at x0-1,
 // P_+1 at x0+128) are computed on the CUDA cores from staged halo sites.
-// CTAs are persistent (4 per SM) and loop over tiles.
+// A CTA takes a contiguous range of the tiles in the order (x segment, y, z)
+// and walks each column (x0, y) along z: a tile shares the lines of two of its
+// three planes with the tile before, so the planes go through a ring of four
+// slots of three dy lines, one plane copied per tile instead of three (at
+// 128^3 a convolution moves 218 MB from L2 to the SMs; staging all nine lines
+// per tile moved 655 MB).  Two accumulators of 48 columns take turns: while
+// the tensor core works on tile i + 1 and the copy of tile i + 2's plane is in
+// flight, warps 0-3 run the epilogue of tile i.  Warp 4 issues the MMAs and
+// warp 5 computes the rows outside the tile ahead of the epilogue (in the
+// epilogue's warps, or both in one, they lengthen the chain of a tile).
+// At 128^3 (ncu): hidden layer 87 us, input gradient 89, output layer 75,
+// against 121 / 148 / 112 with nine lines staged, multiplied and written in
+// turn per tile; bound now by a tile's chain of waits at 18 warps per SM
+// (~3000 cycles; the MMAs take 24 cycles each, 9 per tile, of the tensor pipe).
 constexpr int kTcRows = 128;                          // sites per tile
+constexpr int kTcThreads = kTcRows + 64;
 constexpr int kTcN = 3 * kC;                          // N: 3 dx x 16 output channels
-constexpr int kTcActBytes = 18 * kTcRows * 16;        // 9 lines x 2 planes
+constexpr int kTcSlots = 4;                           // ring of z planes
+constexpr int kTcLineBytes = 2 * kTcRows * 16;        // one line: 2 channel planes
+constexpr int kTcActBytes = kTcSlots * 3 * kTcLineBytes;
 constexpr int kTcWtBytes = 9 * 2 * kTcN * 16;         // 9 lines x 2 planes x 48 rows
-constexpr int kTcHaloBytes = 2 * 9 * 2 * 16;          // x0-1 and x0+128: 9 lines x 2 planes
-constexpr int kTcXchBytes = (2 * 4 + 2) * kC * 4;     // warp-boundary and edge rows (FP32)
+constexpr int kTcHaloBytes = kTcSlots * 3 * 2 * 2 * 16;  // x0-1 and x0+128: [slot][dy][side][plane]
+constexpr int kTcXchBytes = (2 * 4 + 4) * kC * 4;     // warp-boundary rows, two sets of edge rows (FP32)
 constexpr int kTcSmem = kTcActBytes + kTcWtBytes + kTcHaloBytes + kTcXchBytes + 16;
-constexpr int kTcCtasPerSm = 4;
+constexpr int kTcCtasPerSm = 3;
+constexpr int kTcCols = 128;                          // tensor-memory columns: 2 accumulators, 64 apart
 static_assert(kTcCtasPerSm * (kTcSmem + 1024) <= 228 * 1024, "conv CTAs per SM");
+static_assert(kTcCtasPerSm * kTcCols <= 512, "tensor memory of the conv CTAs");
 constexpr unsigned kTcSpin = 1u << 24;                // mbarrier polls before giving up
 
 // tcgen05.mma instruction descriptor: BF16 A and B (K-major), FP32 D, M 128, N 48
@@ -190,6 +216,12 @@ __device__ __forceinline__ void cp16(void* dst_smem, const void* src) {
 }
 __device__ __forceinline__ void cp_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 __device__ __forceinline__ bool tc_try_wait(uint32_t mbar, uint32_t phase) {
@@ -215,34 +247,31 @@ __device__ __forceinline__ int tc_flat(const NetGeom& g, int x, int y, int z) {
   return ((x + y + z) & 1) * g.nh + site_index(x, y, z, g.hx, g.nxy);
 }
 
-// x-line tile t -> (x0, y, z)
-__device__ __forceinline__ void tc_tile(const NetGeom& g, int t, int& x0, int& y, int& z) {
-  const int segs = g.L1 >> 7;
-  x0 = (t % segs) << 7;
-  t /= segs;
-  y = t % g.L2;
-  z = t / g.L2;
+// the tiles of CTA b of n: [first, last) of the order (x segment, y, z)
+__device__ __forceinline__ void tc_range(int ntiles, int& first, int& last) {
+  first = (int)((long long)ntiles * blockIdx.x / gridDim.x);
+  last = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128) conv_tc_kernel(const __nv_bfloat16* __restrict__ in,
+__global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) conv_tc_kernel(const __nv_bfloat16* __restrict__ in,
                                                       const __nv_bfloat16* __restrict__ W,
                                                       const float* __restrict__ bias,
                                                       __nv_bfloat16* __restrict__ out16, float* __restrict__ out32,
                                                       const __nv_bfloat16* __restrict__ mask_src, NetGeom g,
                                                       unsigned* status) {
   extern __shared__ __align__(1024) uint8_t tc_sm[];
-  uint8_t* act = tc_sm;
+  uint8_t* act = tc_sm;                                      // [slot][dy][plane][row] 16 B
   uint8_t* wts = act + kTcActBytes;
-  uint8_t* halo = wts + kTcWtBytes;                          // [side][line][plane] 16 B
-  float* xch = reinterpret_cast<float*>(halo + kTcHaloBytes);  // [0..3] P_-1 of lane 31, [4..7] P_+1 of lane 0, [8] edge lo, [9] edge hi
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(xch + (2 * 4 + 2) * kC);
+  uint8_t* halo = wts + kTcWtBytes;                          // [slot][dy][side][plane] 16 B
+  float* xch = reinterpret_cast<float*>(halo + kTcHaloBytes);  // [0..3] P_-1 of lane 31, [4..7] P_+1 of lane 0, [8 + 2 (i % 2) + side] edges of tile i
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(xch + (2 * 4 + 4) * kC);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ntiles = (g.L1 >> 7) * g.L2 * g.L3;
+  const bool epi = warp < 4;
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(64)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(kTcCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -263,84 +292,134 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const __nv_bfloat16* __res
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
   const uint4* in4 = reinterpret_cast<const uint4*>(in);
-  const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(wts);
-  const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(halo);
   uint32_t phase = 0;
-
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    int x0, y, z;
-    tc_tile(g, t, x0, y, z);
-    // line s = (dy, dz), plane c, row r = site x0 + r; halo sites x0-1, x0+128
+  const int side = lane >> 4;  // warp 5: lane (side, output) of the rows outside the tile
+  float bs[kC];
 #pragma unroll
-    for (int sg = 0; sg < 9; ++sg) {
-      const int yy = wrap(y + sg / 3 - 1, g.L2), zz = wrap(z + sg % 3 - 1, g.L3);
-      const size_t f = (size_t)tc_flat(g, x0 + tid, yy, zz) * 2;
-      cp16(reinterpret_cast<uint4*>(act) + (sg * 2) * kTcRows + tid, in4 + f);
-      cp16(reinterpret_cast<uint4*>(act) + (sg * 2 + 1) * kTcRows + tid, in4 + f + 1);
-    }
-    if (tid < 36) {
-      const int side = tid / 18, sg = (tid >> 1) % 9, c = tid & 1;
-      const int yy = wrap(y + sg / 3 - 1, g.L2), zz = wrap(z + sg % 3 - 1, g.L3);
-      const int xx = wrap(side ? x0 + kTcRows : x0 - 1, g.L1);
-      cp16(reinterpret_cast<uint4*>(halo) + tid, in4 + (size_t)tc_flat(g, xx, yy, zz) * 2 + c);
-    }
-    cp_wait_all();
-    // generic-proxy shared-memory writes -> visible to the tensor core (async proxy)
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  for (int c = 0; c < kC; ++c) bs[c] = MODE != 2 ? __ldg(bias + c) : 0.f;
 
-    if (tid == 0) {
-      const uint32_t a0 = smem_u32(act), b0 = smem_u32(wts);
-#pragma unroll 1
+  int t, tend;
+  tc_range((g.L1 >> 7) * g.L2 * g.L3, t, tend);
+  bool ok = true;
+  while (ok && t < tend) {
+    // one column: tiles z0 .. z0 + n - 1; plane p of the run is z0 - 1 + p, in slot p % 4
+    const int col = t / g.L3, z0 = t - col * g.L3, n = min(g.L3 - z0, tend - t);
+    const int x0 = (col / g.L2) << 7, y = col % g.L2;
+    t += n;
+    auto load_plane = [&](int p) {
+      const int slot = p & (kTcSlots - 1);
+      int zz = z0 - 1 + p;
+      zz = zz < 0 ? zz + g.L3 : (zz >= g.L3 ? zz - g.L3 : zz);
+      if (epi) {
+        uint4* d = reinterpret_cast<uint4*>(act + slot * 3 * kTcLineBytes);
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+          const size_t f = (size_t)tc_flat(g, x0 + tid, wrap(y + dy - 1, g.L2), zz) * 2;
+          cp16(d + (dy * 2) * kTcRows + tid, in4 + f);
+          cp16(d + (dy * 2 + 1) * kTcRows + tid, in4 + f + 1);
+        }
+      } else if (warp == 5 && lane < 12) {
+        // the halo sites, copied and read by warp 5 alone
+        const int dy = lane >> 2, sd = (lane >> 1) & 1, c = lane & 1;
+        const int xx = wrap(sd ? x0 + kTcRows : x0 - 1, g.L1);
+        cp16(reinterpret_cast<uint4*>(halo) + slot * 12 + lane,
+             in4 + (size_t)tc_flat(g, xx, wrap(y + dy - 1, g.L2), zz) * 2 + c);
+      }
+    };
+    // tile i's nine MMAs in the order (dy, dz), into accumulator i & 1
+    auto issue = [&](int i) {
+      const uint32_t a0 = smem_u32(act), dst = tmem + (uint32_t)((i & 1) * 64);
+      uint64_t ad[3];
+#pragma unroll
+      for (int dz = 0; dz < 3; ++dz)
+        ad[dz] = tc_desc(a0 + ((i + dz) & (kTcSlots - 1)) * 3 * kTcLineBytes, kTcRows * 16, 128);
+      const uint64_t bd = tc_desc(smem_u32(wts), kTcN * 16, 128);
+#pragma unroll
       for (int sg = 0; sg < 9; ++sg) {
-        const uint64_t ad = tc_desc(a0 + (sg * 2 * kTcRows) * 16, kTcRows * 16, 128);
-        const uint64_t bd = tc_desc(b0 + (sg * 2 * kTcN) * 16, kTcN * 16, 128);
-        const uint32_t acc = sg > 0 ? 1u : 0u;
+        // (the address fields, in 16-byte units, do not carry out of their 14 bits)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem), "l"(ad), "l"(bd), "r"(kTcIdesc), "r"(acc)
+            ::"r"(dst), "l"(ad[sg % 3] + (uint64_t)(sg / 3 * (kTcLineBytes / 16))), "l"(bd + (uint64_t)(sg * 2 * kTcN)),
+              "r"(kTcIdesc), "r"(sg > 0 ? 1u : 0u)
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        smem_u32(mbar))
                    : "memory");
-    }
-    if (warp == 1) {
-      // the rows outside the tile on the CUDA cores: lanes 0-15 P_-1[x0-1][o],
-      // lanes 16-31 P_+1[x0+128][o]
-      const int side = lane >> 4, o = lane & 15, n = (side ? 2 : 0) * kC + o;
-      float v = 0.f;
-#pragma unroll 1
-      for (int sg = 0; sg < 9; ++sg) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const __nv_bfloat16* xr = hb + ((side * 9 + sg) * 2 + c) * 8;
-          const __nv_bfloat16* wr = wb + ((size_t)(sg * 2 + c) * kTcN + n) * 8;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v = fmaf(__bfloat162float(xr[q]), __bfloat162float(wr[q]), v);
-        }
-      }
-      xch[(8 + side) * kC + o] = v;
-    }
-    const uint32_t ph = phase;
-    phase ^= 1u;
-    const bool done = tc_wait(smem_u32(mbar), ph);
-    if (__syncthreads_or(!done)) {
-      // record the failure, give the MMAs a second bounded wait, then stop
-      if (!done) {
-        if (lane == 0) atomicOr(status, 1u);
-        tc_wait(smem_u32(mbar), ph);
-      }
-      break;
-    }
+    };
+    load_plane(0);
+    load_plane(1);
+    load_plane(2);
+    cp_commit();
+    if (n > 1) load_plane(3);
+    cp_commit();
+    cp_wait<1>();
+    // generic-proxy shared-memory writes -> visible to the tensor core (async proxy)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // row j = 32 warp + lane: P_-1[j] (columns 0-15), P_0[j] (16-31), P_+1[j] (32-47)
-    uint32_t vm[16], v0[16], vp[16];
-    const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
+    if (tid == kTcRows) issue(0);
+
+    for (int i = 0; i < n; ++i) {
+      const int f = epi ? tc_flat(g, x0 + tid, y, z0 + i) : 0;
+      uint4 m0, m1;  // MODE 2: the activation whose sign masks the gradient
+      if (MODE == 2 && epi) {
+        const uint4* m = reinterpret_cast<const uint4*>(mask_src) + (size_t)f * 2;
+        m0 = __ldg(m);
+        m1 = __ldg(m + 1);
+      }
+      if (warp == 5) {
+        // the rows outside tile i on the CUDA cores: lanes 0-15 P_-1[x0-1][o],
+        // lanes 16-31 P_+1[x0+128][o] (the tile's planes were waited for before its MMAs)
+        float v = 0.f;
+#pragma unroll
+        for (int sg = 0; sg < 9; ++sg) {
+          const int slot = (i + sg % 3) & (kTcSlots - 1);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const uint4 x = reinterpret_cast<const uint4*>(halo)[((slot * 3 + sg / 3) * 2 + side) * 2 + c];
+            const uint4 w = reinterpret_cast<const uint4*>(wts)[(sg * 2 + c) * kTcN + side * 2 * kC + (lane & 15)];
+            const uint32_t xw[4] = {x.x, x.y, x.z, x.w}, ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              v = fmaf(bf_lo(xw[q]), bf_lo(ww[q]), v);
+              v = fmaf(bf_hi(xw[q]), bf_hi(ww[q]), v);
+            }
+          }
+        }
+        xch[(8 + 2 * (i & 1) + side) * kC + (lane & 15)] = v;
+        __syncwarp();
+      }
+      const uint32_t ph = phase;
+      phase ^= 1u;
+      const bool done = tc_wait(smem_u32(mbar), ph);
+      // tile i's MMAs have read slot i % 4 (plane i) for the last time
+      if (done && i + 2 < n) load_plane(i + 4);
+      cp_commit();
+      cp_wait<1>();  // the planes of tile i + 1
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      if (__syncthreads_or(!done)) {
+        // record the failure, give the MMAs a second bounded wait, then stop
+        if (!done) {
+          if (lane == 0) atomicOr(status, 1u);
+          tc_wait(smem_u32(mbar), ph);
+        }
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!epi) {
+        if (tid == kTcRows && i + 1 < n) issue(i + 1);
+        __syncwarp();
+        continue;
+      }
+      // row j = 32 warp + lane: P_-1[j] (columns 0-15), P_0[j] (16-31), P_+1[j] (32-47)
+      uint32_t vm[16], v0[16], vp[16];
+      const uint32_t ta = tmem + (uint32_t)((i & 1) * 64) + ((uint32_t)(warp * 32) << 16);
 #define LCE_TC_LD16(dst, col)                                                                                   \
   asm volatile(                                                                                                 \
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, " \
@@ -349,67 +428,72 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const __nv_bfloat16* __res
         "=r"(dst[7]), "=r"(dst[8]), "=r"(dst[9]), "=r"(dst[10]), "=r"(dst[11]), "=r"(dst[12]), "=r"(dst[13]),   \
         "=r"(dst[14]), "=r"(dst[15])                                                                            \
       : "r"(ta + (col)))
-    LCE_TC_LD16(vm, 0);
-    LCE_TC_LD16(v0, 16);
-    LCE_TC_LD16(vp, 32);
+      LCE_TC_LD16(vm, 0);
+      LCE_TC_LD16(v0, 16);
+      LCE_TC_LD16(vp, 32);
 #undef LCE_TC_LD16
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    // rows across warp boundaries
-    if (lane == 31) {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      // rows across warp boundaries
+      if (lane == 31 || lane == 0) {
+        uint4* d = reinterpret_cast<uint4*>(xch + (lane ? warp : 4 + warp) * kC);
 #pragma unroll
-      for (int c = 0; c < kC; ++c) xch[warp * kC + c] = __uint_as_float(vm[c]);
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int c = 0; c < kC; ++c) xch[(4 + warp) * kC + c] = __uint_as_float(vp[c]);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    const float* lo = lane == 0 ? (warp == 0 ? xch + 8 * kC : xch + (warp - 1) * kC) : nullptr;
-    const float* hi = lane == 31 ? (warp == 3 ? xch + 9 * kC : xch + (4 + warp + 1) * kC) : nullptr;
-    float o[kC];
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      const float pm = __shfl_up_sync(0xffffffffu, __uint_as_float(vm[c]), 1);
-      const float pp = __shfl_down_sync(0xffffffffu, __uint_as_float(vp[c]), 1);
-      o[c] = (lo ? lo[c] : pm) + __uint_as_float(v0[c]) + (hi ? hi[c] : pp) + (MODE != 2 ? bias[c] : 0.f);
-    }
-    const int f = tc_flat(g, x0 + tid, y, z);
-    if (MODE == 1) {
-      float4* d = reinterpret_cast<float4*>(out32 + (size_t)f * 8);
-      d[0] = make_float4(o[0], o[1], o[2], o[3]);
-      d[1] = make_float4(o[4], o[5], o[6], o[7]);
-    } else {
-      if (MODE == 0) {
-#pragma unroll
-        for (int c = 0; c < kC; ++c) o[c] = fmaxf(o[c], 0.f);
-      } else {
-        const __nv_bfloat16* m = mask_src + (size_t)f * kC;
-#pragma unroll
-        for (int c = 0; c < kC; ++c)
-          if (!(__bfloat162float(m[c]) > 0.f)) o[c] = 0.f;
+        for (int c = 0; c < 4; ++c)
+          d[c] = lane ? make_uint4(vm[4 * c], vm[4 * c + 1], vm[4 * c + 2], vm[4 * c + 3])
+                      : make_uint4(vp[4 * c], vp[4 * c + 1], vp[4 * c + 2], vp[4 * c + 3]);
       }
-      uint4 w0, w1;
-      w0.x = pack2(__float2bfloat16_rn(o[0]), __float2bfloat16_rn(o[1]));
-      w0.y = pack2(__float2bfloat16_rn(o[2]), __float2bfloat16_rn(o[3]));
-      w0.z = pack2(__float2bfloat16_rn(o[4]), __float2bfloat16_rn(o[5]));
-      w0.w = pack2(__float2bfloat16_rn(o[6]), __float2bfloat16_rn(o[7]));
-      w1.x = pack2(__float2bfloat16_rn(o[8]), __float2bfloat16_rn(o[9]));
-      w1.y = pack2(__float2bfloat16_rn(o[10]), __float2bfloat16_rn(o[11]));
-      w1.z = pack2(__float2bfloat16_rn(o[12]), __float2bfloat16_rn(o[13]));
-      w1.w = pack2(__float2bfloat16_rn(o[14]), __float2bfloat16_rn(o[15]));
-      uint4* d = reinterpret_cast<uint4*>(out16) + (size_t)f * 2;
-      d[0] = w0;
-      d[1] = w1;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(kTcRows) : "memory");  // warps 0-3
+      float o[kC];
+#pragma unroll
+      for (int c = 0; c < kC; ++c) {
+        float pm = __shfl_up_sync(0xffffffffu, __uint_as_float(vm[c]), 1);
+        float pp = __shfl_down_sync(0xffffffffu, __uint_as_float(vp[c]), 1);
+        vm[c] = __float_as_uint(pm);
+        vp[c] = __float_as_uint(pp);
+      }
+      if (lane == 31 || lane == 0) {
+        const int edge = 8 + 2 * (i & 1);
+        const uint4* e = reinterpret_cast<const uint4*>(
+            xch + (lane == 0 ? (warp == 0 ? edge : warp - 1) : (warp == 3 ? edge + 1 : 4 + warp + 1)) * kC);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint4 r = e[c];
+          if (lane == 0) vm[4 * c] = r.x, vm[4 * c + 1] = r.y, vm[4 * c + 2] = r.z, vm[4 * c + 3] = r.w;
+          else vp[4 * c] = r.x, vp[4 * c + 1] = r.y, vp[4 * c + 2] = r.z, vp[4 * c + 3] = r.w;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < kC; ++c)
+        o[c] = __uint_as_float(vm[c]) + __uint_as_float(v0[c]) + __uint_as_float(vp[c]) + (MODE != 2 ? bs[c] : 0.f);
+      if (MODE == 1) {
+        float4* d = reinterpret_cast<float4*>(out32 + (size_t)f * 8);
+        d[0] = make_float4(o[0], o[1], o[2], o[3]);
+        d[1] = make_float4(o[4], o[5], o[6], o[7]);
+      } else {
+        if (MODE == 0) {
+#pragma unroll
+          for (int c = 0; c < kC; ++c) o[c] = fmaxf(o[c], 0.f);
+        } else {
+          const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+          for (int c = 0; c < kC; ++c)
+            if (!((c & 1 ? bf_hi(mw[c >> 1]) : bf_lo(mw[c >> 1])) > 0.f)) o[c] = 0.f;
+        }
+        const uint4 w0 = make_uint4(pack2f(o[0], o[1]), pack2f(o[2], o[3]), pack2f(o[4], o[5]), pack2f(o[6], o[7]));
+        const uint4 w1 =
+            make_uint4(pack2f(o[8], o[9]), pack2f(o[10], o[11]), pack2f(o[12], o[13]), pack2f(o[14], o[15]));
+        uint4* d = reinterpret_cast<uint4*>(out16) + (size_t)f * 2;
+        d[0] = w0;
+        d[1] = w1;
+      }
     }
-    // the exchange rows, the staged tile and the accumulator are reused by the next tile
-    __syncthreads();
   }
+  cp_wait<0>();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
   }
 }
 
@@ -633,27 +717,42 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __nv_bfloat16* __restr
 }
 
 // grad W[k][co][ci] = sum over chunks of part (blocks 0..26); grad b[co]
-// (block 27) -- fixed summation order, so the gradient is deterministic
-__global__ void wgrad_sum_kernel(const float* part, int nchunk, float* gW) {
-  const int k = blockIdx.x, e = threadIdx.x;  // 256 threads
+// (block 27) -- fixed summation order, so the gradient is deterministic.
+// A round trip to L2 per batch of loads sets its time: 32 loads in flight
+// before their in-order adds, one warp per block over the whole chip (17 us
+// for 592 partials; 27 us with 28 blocks of 256 threads).
+__device__ __forceinline__ float chunk_sum(const float* p, int stride, int nchunk) {
+  constexpr int kBatch = 32;
   float s = 0.f;
+  for (int c = 0; c < nchunk; c += kBatch) {
+    float v[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) v[j] = c + j < nchunk ? __ldg(p + (size_t)(c + j) * stride) : 0.f;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j)
+      if (c + j < nchunk) s += v[j];
+  }
+  return s;
+}
+__global__ void __launch_bounds__(32) wgrad_sum_kernel(const float* part, int nchunk, float* gW) {
+  const int k = blockIdx.x, e = blockIdx.y * 32 + threadIdx.x;
   if (k < kK) {
-    for (int c = 0; c < nchunk; ++c) s += part[((size_t)k * nchunk + c) * kC * kC + e];
-    gW[(size_t)k * kC * kC + e] = s;
+    gW[(size_t)k * kC * kC + e] = chunk_sum(part + (size_t)k * nchunk * kC * kC + e, kC * kC, nchunk);
   } else if (e < kC) {
-    const float* bp = part + (size_t)kK * nchunk * kC * kC;
-    for (int c = 0; c < nchunk; ++c) s += bp[(size_t)c * kC + e];
-    gW[(size_t)kK * kC * kC + e] = s;
+    gW[(size_t)kK * kC * kC + e] = chunk_sum(part + (size_t)kK * nchunk * kC * kC + e, kC, nchunk);
   }
 }
 
-// loss 1 - q . t per site, q = o/|o|; gz = dL/do = -(t - (q.t) q) / (|o| N)
+// loss 1 - q . t per site, q = o/|o|; gz = dL/do = -(t - (q.t) q) / (|o| N).
+// One 16-byte access per record (o: the first half of its 32 bytes, t; gz two):
+// 23 us at 128^3, 51 us with 4-byte accesses.
 __global__ void loss_kernel(const float* out, const float* target, int nsites, __nv_bfloat16* gz, double* part) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double l[1] = {0.0};
   if (i < nsites) {
-    const float* o = out + (size_t)i * 8;
-    const float* t = target + (size_t)i * 4;
+    const float4 o4 = __ldg(reinterpret_cast<const float4*>(out) + 2 * (size_t)i);
+    const float4 t4 = __ldg(reinterpret_cast<const float4*>(target) + i);
+    const float o[4] = {o4.x, o4.y, o4.z, o4.w}, t[4] = {t4.x, t4.y, t4.z, t4.w};
     const float n = sqrtf(o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3]) + 1e-12f;
     float q[4], qt = 0.f;
     for (int c = 0; c < 4; ++c) {
@@ -662,10 +761,10 @@ __global__ void loss_kernel(const float* out, const float* target, int nsites, _
     }
     l[0] = 1.0 - qt;
     const float sc = -1.0f / (n * (float)nsites);
-    uint32_t* gz32 = reinterpret_cast<uint32_t*>(gz) + (size_t)i * 8;
-    gz32[0] = pack2(__float2bfloat16_rn(sc * (t[0] - qt * q[0])), __float2bfloat16_rn(sc * (t[1] - qt * q[1])));
-    gz32[1] = pack2(__float2bfloat16_rn(sc * (t[2] - qt * q[2])), __float2bfloat16_rn(sc * (t[3] - qt * q[3])));
-    for (int w = 2; w < 8; ++w) gz32[w] = 0u;
+    uint4* g4 = reinterpret_cast<uint4*>(gz) + 2 * (size_t)i;
+    g4[0] = make_uint4(pack2f(sc * (t[0] - qt * q[0]), sc * (t[1] - qt * q[1])),
+                       pack2f(sc * (t[2] - qt * q[2]), sc * (t[3] - qt * q[3])), 0u, 0u);
+    g4[1] = make_uint4(0u, 0u, 0u, 0u);
   }
   block_reduce_store<1>(l, part + blockIdx.x);
 }
@@ -675,13 +774,13 @@ __global__ void loss_kernel(const float* out, const float* target, int nsites, _
 __global__ void refresh_kernel(float* w32, __nv_bfloat16* w16, __nv_bfloat16* wt16) {
   const int l = blockIdx.x;
   float* W = w32 + (size_t)l * kPl;
-  for (int e = threadIdx.x; e < kWl; e += blockDim.x) {
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < kWl; e += gridDim.y * blockDim.x) {
     const int k = e / (kC * kC), co = (e / kC) % kC, ci = e % kC;
     if (l == kLayers - 1 && co >= kOut) W[e] = 0.f;
     w16[(size_t)l * kWl + e] = __float2bfloat16_rn(W[e]);
     wt16[(size_t)l * kWl + ((size_t)(kK - 1 - k) * kC + ci) * kC + co] = __float2bfloat16_rn(W[e]);
   }
-  if (l == kLayers - 1 && threadIdx.x >= kOut && threadIdx.x < kC) W[kWl + threadIdx.x] = 0.f;
+  if (blockIdx.y == 0 && l == kLayers - 1 && threadIdx.x >= kOut && threadIdx.x < kC) W[kWl + threadIdx.x] = 0.f;
 }
 
 __global__ void adam_kernel(float* w, float* m, float* v, const float* grad, int n, float lr, float b1, float b2,
@@ -820,7 +919,6 @@ int net_fail(lce_net* n, int code, const std::string& m) {
 // shared memory; tensor memory: 4 x 128 columns).  The runtime's occupancy
 // query reported 1 per SM for this kernel where the launch itself holds 4.
 static_assert(kTgMaxCtasPerSm * (kTgSmem + 1024) <= 228 * 1024, "wgrad CTAs per SM");
-static_assert(kTcCtasPerSm == kTgMaxCtasPerSm, "the convolution uses the weight gradient's grid");
 template <typename K>
 void tc_attributes(K kernel, int smem) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -877,58 +975,58 @@ int conv_grid(long nsites) {
   return std::max(1, std::min(ceil_div(ntiles, kConvWarps), 148 * 8));
 }
 
-// forward through all layers from act[0]; output in n->out
+// forward through all layers from x (act[0], or a recorded pair's features); output in n->out
 // one convolution: the tcgen05 kernel when L1 is a multiple of 128, else the
 // mma.sync kernel
 template <int MODE>
 void launch_conv(lce_net* n, const __nv_bfloat16* in, const __nv_bfloat16* W, const float* bias,
                  __nv_bfloat16* out16, float* out32, const __nv_bfloat16* mask, const NetGeom& g, cudaStream_t s) {
   if (g.L1 % 128 == 0) {
-    // persistent CTAs, 4 per SM, like the weight gradient
-    const int grid = std::min(wgrad_tc_grid(n), (g.L1 / 128) * g.L2 * g.L3);
-    conv_tc_kernel<MODE><<<grid, 128, kTcSmem, s>>>(in, W, bias, out16, out32, mask, g, n->flag);
+    // persistent CTAs, kTcCtasPerSm per SM
+    const int grid = std::min(wgrad_tc_grid(n) / kTgMaxCtasPerSm * kTcCtasPerSm, (g.L1 / 128) * g.L2 * g.L3);
+    conv_tc_kernel<MODE><<<grid, kTcThreads, kTcSmem, s>>>(in, W, bias, out16, out32, mask, g, n->flag);
   } else {
     conv_kernel<MODE><<<conv_grid(2L * g.nh), 32 * kConvWarps, 0, s>>>(in, W, bias, out16, out32, mask, g);
   }
 }
 
-void net_forward(lce_net* n, const NetGeom& g, cudaStream_t s) {
+void net_forward(lce_net* n, const __nv_bfloat16* x, const NetGeom& g, cudaStream_t s) {
   for (int l = 0; l < kLayers; ++l) {
     const __nv_bfloat16* W = n->w16 + (size_t)l * kWl;
     const float* b = n->w32 + (size_t)l * kPl + kWl;
-    if (l < kLayers - 1) launch_conv<0>(n, n->act[l], W, b, n->act[l + 1], nullptr, nullptr, g, s);
-    else launch_conv<1>(n, n->act[l], W, b, nullptr, n->out, nullptr, g, s);
+    const __nv_bfloat16* in = l ? n->act[l] : x;
+    if (l < kLayers - 1) launch_conv<0>(n, in, W, b, n->act[l + 1], nullptr, nullptr, g, s);
+    else launch_conv<1>(n, in, W, b, nullptr, n->out, nullptr, g, s);
   }
 }
 
-// loss and gradients (into n->grad) for act[0] and n->target; returns the
-// loss through part (device) -- caller sums
-void net_backward(lce_net* n, const NetGeom& g, cudaStream_t s) {
+// loss and gradients (into n->grad) for the input x and the target t; returns
+// the loss through part (device) -- caller sums
+void net_backward(lce_net* n, const __nv_bfloat16* x, const float* t, const NetGeom& g, cudaStream_t s) {
   const long ns = 2L * g.nh;
-  loss_kernel<<<ceil_div(ns, 256), 256, 0, s>>>(n->out, n->target, (int)ns, n->gz, n->part);
+  loss_kernel<<<ceil_div(ns, 256), 256, 0, s>>>(n->out, t, (int)ns, n->gz, n->part);
   __nv_bfloat16* gz = n->gz;   // gradient at the output of layer l (pre-activation)
   __nv_bfloat16* gy = n->gy;
   for (int l = kLayers - 1; l >= 0; --l) {
     float* gW = n->grad + (size_t)l * kPl;
+    const __nv_bfloat16* in = l ? n->act[l] : x;
     if (g.L1 % 128 == 0) {
       const int grid = std::min(wgrad_tc_grid(n), (g.L1 / 128) * g.L2 * g.L3);
-      wgrad_tc_kernel<<<grid, 128, kTgSmem, s>>>(gz, n->act[l], n->wpart, grid, g, n->flag);
-      wgrad_sum_kernel<<<kK + 1, kC * kC, 0, s>>>(n->wpart, grid, gW);
+      wgrad_tc_kernel<<<grid, 128, kTgSmem, s>>>(gz, in, n->wpart, grid, g, n->flag);
+      wgrad_sum_kernel<<<dim3(kK + 1, kC * kC / 32), 32, 0, s>>>(n->wpart, grid, gW);
     } else {
-      wgrad_kernel<<<dim3(n->nchunk, kK), 128, 0, s>>>(gz, n->act[l], n->wpart, n->nchunk, g);
-      wgrad_sum_kernel<<<kK + 1, kC * kC, 0, s>>>(n->wpart, n->nchunk, gW);
+      wgrad_kernel<<<dim3(n->nchunk, kK), 128, 0, s>>>(gz, in, n->wpart, n->nchunk, g);
+      wgrad_sum_kernel<<<dim3(kK + 1, kC * kC / 32), 32, 0, s>>>(n->wpart, n->nchunk, gW);
     }
     if (l > 0) {
       // gradient w.r.t. act[l] = conv_T(gz, W_l), times relu'(layer l-1) = (act[l] > 0)
       launch_conv<2>(n, gz, n->wt16 + (size_t)l * kWl, nullptr, gy, nullptr, n->act[l], g, s);
-      __nv_bfloat16* t = gz;
-      gz = gy;
-      gy = t;
+      std::swap(gz, gy);
     }
   }
 }
 
-void net_refresh(lce_net* n, cudaStream_t s) { refresh_kernel<<<kLayers, 256, 0, s>>>(n->w32, n->w16, n->wt16); }
+void net_refresh(lce_net* n, cudaStream_t s) { refresh_kernel<<<dim3(kLayers, kWl / 256), 256, 0, s>>>(n->w32, n->w16, n->wt16); }
 
 }  // namespace
 
@@ -1057,8 +1155,8 @@ int lce_net_eval(lce_net* n, int L1, int L2, int L3, const float* feat, const fl
   for (size_t i = 0; i < fb.size(); ++i) fb[i] = __bfloat16_as_ushort(__float2bfloat16_rn(feat[i]));
   NCK(cudaMemcpyAsync(n->act[0], fb.data(), fb.size() * 2, cudaMemcpyHostToDevice, n->stream));
   NCK(cudaMemcpyAsync(n->target, target, sizeof(float) * ns * 4, cudaMemcpyHostToDevice, n->stream));
-  net_forward(n, g, n->stream);
-  net_backward(n, g, n->stream);
+  net_forward(n, n->act[0], g, n->stream);
+  net_backward(n, n->act[0], n->target, g, n->stream);
   NCK(cudaGetLastError());
   std::vector<double> lp(ceil_div(ns, 256));
   NCK(cudaMemcpyAsync(lp.data(), n->part, lp.size() * sizeof(double), cudaMemcpyDeviceToHost, n->stream));
@@ -1112,10 +1210,8 @@ int lce_net_train(lce_net* n, int epochs, double lr, double* mean_loss) {
       const long ns = 2L * p.g.nh;
       int rc = net_buffers(n, ns);
       if (rc) return rc;
-      NCK(cudaMemcpyAsync(n->act[0], p.feat, (size_t)ns * kC * 2, cudaMemcpyDeviceToDevice, n->stream));
-      NCK(cudaMemcpyAsync(n->target, p.target, (size_t)ns * 16, cudaMemcpyDeviceToDevice, n->stream));
-      net_forward(n, p.g, n->stream);
-      net_backward(n, p.g, n->stream);
+      net_forward(n, p.feat, p.g, n->stream);
+      net_backward(n, p.feat, p.target, p.g, n->stream);
       ++n->step;
       const float c1 = 1.f - std::pow(b1, (float)n->step), c2 = 1.f - std::pow(b2, (float)n->step);
       adam_kernel<<<64, 256, 0, n->stream>>>(n->w32, n->m, n->v, n->grad, kNParam, (float)lr, b1, b2, eps, c1, c2);
@@ -1150,7 +1246,7 @@ int net_features(lce_net* n, const ChainDev* chd, const ChainDev& ch, bool f64, 
 }
 
 void net_predict(lce_net* n, const ChainDev& ch, cudaStream_t s) {
-  net_forward(n, make_geom(ch.L1, ch.L2, ch.L3), s);
+  net_forward(n, n->act[0], make_geom(ch.L1, ch.L2, ch.L3), s);
 }
 
 // ch.g = Omega G_prev from the last net_predict

@@ -56,6 +56,15 @@ def test_forward_loss_gradient_match_fp64_reference(L):
     assert np.array_equal(out, out2) and np.array_equal(grad, grad2) and loss == loss2
 
 
+# more tiles than the tcgen05 kernels' CTAs hold at once, so that a CTA walks
+# part of one column and part of the next (L3 odd against the split, one and
+# two x segments, the shortest column); the reference and the tolerances of
+# the test above
+@pytest.mark.parametrize("L", [(128, 40, 26), (256, 14, 34), (128, 500, 2)])
+def test_long_columns_match_fp64_reference(L):
+    test_forward_loss_gradient_match_fp64_reference(L)
+
+
 def test_untrained_network_is_identity_and_params_roundtrip(tmp_path):
     from lceqcd_b200 import GaugeNet
     net = GaugeNet(seed=7)
