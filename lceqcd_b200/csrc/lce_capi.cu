@@ -380,7 +380,8 @@ int enq_pass(lce_ctx* c, Enq& q, size_t i) {
   const int nblocks = q.blk->back();
   const bool reduce = q.measflag == 1 || ps.kind == kHiggsMetro;
   if (reduce && q.slot >= c->part_slots) return fail(c, LCE_ERR_INVALID, "too many reduction slots");
-  PassArgs a{};
+  PassArgsMany a;
+  static_cast<PassArgs&>(a) = PassArgs{};
   a.chains = c->ch_d;
   a.blk_begin = q.blk_d;
   a.spt = q.spt;
@@ -394,6 +395,12 @@ int enq_pass(lce_ctx* c, Enq& q, size_t i) {
   a.stream_off = q.soff;
   a.pass_off = q.poff;
   a.nchains = c->nchains;
+  a.many = c->nchains > 1 && c->nchains <= kParamChains && nblocks >= kParamTiles;
+  a.ch[0] = c->ch[0];
+  if (a.many) {
+    std::copy(c->ch.begin(), c->ch.end(), a.ch);
+    std::copy(q.blk->begin(), q.blk->end(), a.begin);
+  }
   a.eo = ps.eo ^ c->eo_flip;
   a.fuse_renorm = q.fuse ? 1 : 0;
   a.s_lo = c->s_lo;

@@ -184,6 +184,26 @@ struct PassArgs {
   // 64-register kernels.)
   int ntiles, rb_slot, rb_nitems;
 };
+// with a single-chain context's chain, for the kernels that read it from the
+// parameter bank (lce_update.cu: ONE)
+struct PassArgsOne : PassArgs {
+  ChainDev one;
+  // its couplings in FP32 (FP32 contexts)
+  float beta, beta_a, beta_2, beta_4, inv_beta2, cxval0;
+};
+
+// with the chains of a batch: the table and the tiles of a pass before each
+// chain in the parameter bank too (many = 1), for a batch of at most
+// kParamChains chains (22.5 KB of arguments) and at least kParamTiles tiles
+// per pass.  Below that a pass is launch-bound and the larger argument block
+// costs more than it gives (2 chains of 8^3: 29.4 -> 30.6 us per sweep, 12 of
+// 16^3, 192 tiles: 35.0 -> 35.7; 24 of 16^3-32^3, 1584 tiles: 85.3 -> 81.9).
+constexpr int kParamChains = 128, kParamTiles = 512;
+struct PassArgsMany : PassArgs {
+  int many;
+  ChainDev ch[kParamChains];
+  int begin[kParamChains + 1];
+};
 
 struct FinalizeArgs {
   const ChainDev* chains;
@@ -238,14 +258,14 @@ int persistent_grid();  // co-resident blocks of the persistent kernel on this d
 template <typename R>
 cudaError_t launch_persistent(const PersistArgs& a, int grid, cudaStream_t s);
 template <typename R>
-void launch_higgs(int mode, const PassArgs& a, int nblocks, cudaStream_t s);
+void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s);
 template <typename R>
-void launch_link(int mode, int mu, const PassArgs& a, int nblocks, cudaStream_t s);
+void launch_link(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStream_t s);
 void launch_finalize(const FinalizeArgs& f, cudaStream_t s);
 // a sweep's first pass (ahiggs2, eo 0) with one extra block running the
 // previous sweep's single-chain finalize fp (graphs of several sweeps)
 template <typename R>
-void launch_higgs_fin(const PassArgs& a, const FinalizeArgs& fp, int nblocks, cudaStream_t s);
+void launch_higgs_fin(const PassArgsMany& a, const FinalizeArgs& fp, int nblocks, cudaStream_t s);
 template <typename R>
 void launch_renorm(void* u, size_t nlinks, cudaStream_t s);
 template <typename R>

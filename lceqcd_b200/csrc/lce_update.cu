@@ -29,6 +29,7 @@
 // (site, call, pass), or, in validation mode, the host-supplied stream indexed
 // in the reference's consumption order (slot layouts in lce_common.cuh).
 #include <algorithm>
+#include <type_traits>
 
 #include "lce_internal.hpp"
 
@@ -55,15 +56,72 @@ __device__ __forceinline__ int find_chain(const int* blk_begin, int n, int b) {
 // loads are not enough there: measured on B200, lines an SM's L1 fetched
 // before the barrier were still served after it (the persistent sweep then
 // differs from the per-pass sweep), so L1 is bypassed.
+//
+// ONE not kTable (the chain in the parameter bank): a plane's base is one address in uniform registers and a load costs
+// one multiply-add of the 32-bit site index.  Otherwise a link's plane and
+// site are added first: a base per plane would take vector registers.
 template <typename R, bool NC = true>
 __device__ __forceinline__ R ldA(const R* A, int nh, int p, int k, int s) {
   const R* q = A + ((size_t)(p * 3 + k)) * nh + s;
   return NC ? __ldg(q) : __ldcg(q);
 }
 
-template <typename R, bool NC = true>
+// A pass kernel's arguments, by where it finds the chain its block works on.
+enum Chains : int { kTable = 0, kOne = 1, kMany = 2 };
+template <int ONE>
+using Args = std::conditional_t<ONE == kOne, PassArgsOne, std::conditional_t<ONE == kMany, PassArgsMany, PassArgs>>;
+__device__ __forceinline__ const ChainDev& chain_of(const PassArgsOne& p, int) { return p.one; }
+__device__ __forceinline__ const ChainDev& chain_of(const PassArgsMany& p, int c) { return p.ch[c]; }
+__device__ __forceinline__ const ChainDev& chain_of(const PassArgs& p, int c) { return p.chains[c]; }
+// the chain of a block's tile, and the tile's place among the chain's
+__device__ __forceinline__ int find_tile(const PassArgsOne&, int&) { return 0; }
+__device__ __forceinline__ int find_tile(const PassArgsMany& p, int& tile) {
+  int lo = 0, hi = p.nchains - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (p.begin[mid] <= tile) lo = mid;
+    else hi = mid - 1;
+  }
+  tile -= p.begin[lo];
+  return lo;
+}
+__device__ __forceinline__ int find_tile(const PassArgs& p, int& tile) {
+  const int c = p.nchains > 1 ? find_chain(p.blk_begin, p.nchains, tile) : 0;
+  tile -= __ldg(p.blk_begin + c);
+  return c;
+}
+
+// the couplings in the kernels' precision (FP32, ONE: converted on the host)
+template <typename R, int ONE>
+struct Cpl {
+  const ChainDev& c;
+  __device__ Cpl(const Args<ONE>&, const ChainDev& ch) : c(ch) {}
+  __device__ R beta() const { return (R)c.beta; }
+  __device__ R beta_a() const { return (R)c.beta_a; }
+  __device__ R beta_2() const { return (R)c.beta_2; }
+  __device__ R beta_4() const { return (R)c.beta_4; }
+  __device__ R inv_beta2() const { return (R)c.inv_beta2; }
+  __device__ R cxval0() const { return (R)c.cxval0; }
+};
+template <>
+struct Cpl<float, kOne> {
+  const PassArgsOne& a;
+  __device__ Cpl(const PassArgsOne& p, const ChainDev&) : a(p) {}
+  __device__ float beta() const { return a.beta; }
+  __device__ float beta_a() const { return a.beta_a; }
+  __device__ float beta_2() const { return a.beta_2; }
+  __device__ float beta_4() const { return a.beta_4; }
+  __device__ float inv_beta2() const { return a.inv_beta2; }
+  __device__ float cxval0() const { return a.cxval0; }
+};
+
+template <typename R, bool NC = true, int ONE = kTable>
 __device__ __forceinline__ su2<R> ldU(const ChainDev& ch, int mu, int p, int s) {
-  const size_t i = ((size_t)(mu * 2 + p)) * ch.nh + s;
+  if (ONE != kTable) {
+    const void* plane = static_cast<const char*>(ch.u) + (size_t)(mu * 2 + p) * ch.nh * LinkIO<R>::kBytes;
+    return NC ? LinkIO<R>::ld(plane, s) : LinkIO<R>::ld_cg(plane, s);
+  }
+  const size_t i = (size_t)(mu * 2 + p) * ch.nh + s;
   return NC ? LinkIO<R>::ld(ch.u, i) : LinkIO<R>::ld_cg(ch.u, i);
 }
 
@@ -71,45 +129,45 @@ __device__ __forceinline__ su2<R> ldU(const ChainDev& ch, int mu, int p, int s) 
 //   upper  = U_nu(x+mu) [U_mu(x+nu)^+ U_nu(x)^+]          (NN of DD)
 //   lower  = U_nu(x-nu+mu)^+ [U_mu(x-nu)^+ U_nu(x-nu)]    (DN of DN)
 //   V      = (V + upper) + lower
-template <typename R, int MU, int NU, bool NC>
+template <typename R, int MU, int NU, bool NC, int ONE>
 __device__ __forceinline__ void staple_add(const ChainDev& ch, int eo, const NbrOff& o, int s, su2<R>& V) {
   const int oe = 1 - eo;
   const int xpmu = s + o.p[MU], xpnu = s + o.p[NU], xmnu = s + o.m[NU];
   const int xmnupmu = xmnu + o.p[MU];
-  su2<R> up1 = dd(ldU<R, NC>(ch, MU, oe, xpnu), ldU<R, NC>(ch, NU, eo, s));
-  su2<R> up2 = nn(ldU<R, NC>(ch, NU, oe, xpmu), up1);
-  su2<R> bt1 = dn(ldU<R, NC>(ch, MU, oe, xmnu), ldU<R, NC>(ch, NU, oe, xmnu));
-  su2<R> bt2 = dn(ldU<R, NC>(ch, NU, eo, xmnupmu), bt1);
+  su2<R> up1 = dd(ldU<R, NC, ONE>(ch, MU, oe, xpnu), ldU<R, NC, ONE>(ch, NU, eo, s));
+  su2<R> up2 = nn(ldU<R, NC, ONE>(ch, NU, oe, xpmu), up1);
+  su2<R> bt1 = dn(ldU<R, NC, ONE>(ch, MU, oe, xmnu), ldU<R, NC, ONE>(ch, NU, oe, xmnu));
+  su2<R> bt2 = dn(ldU<R, NC, ONE>(ch, NU, eo, xmnupmu), bt1);
   V.a = (V.a + up2.a) + bt2.a;
   V.b = (V.b + up2.b) + bt2.b;
 }
 
-template <typename R, int MU, bool NC = true>
+template <typename R, int MU, bool NC = true, int ONE = kTable>
 __device__ __forceinline__ su2<R> staple(const ChainDev& ch, int eo, const NbrOff& o, int s) {
   su2<R> V{{(R)0, (R)0}, {(R)0, (R)0}};
   if (MU == 0) {
-    staple_add<R, 0, 1, NC>(ch, eo, o, s, V);
-    staple_add<R, 0, 2, NC>(ch, eo, o, s, V);
+    staple_add<R, 0, 1, NC, ONE>(ch, eo, o, s, V);
+    staple_add<R, 0, 2, NC, ONE>(ch, eo, o, s, V);
   } else if (MU == 1) {
-    staple_add<R, 1, 0, NC>(ch, eo, o, s, V);
-    staple_add<R, 1, 2, NC>(ch, eo, o, s, V);
+    staple_add<R, 1, 0, NC, ONE>(ch, eo, o, s, V);
+    staple_add<R, 1, 2, NC, ONE>(ch, eo, o, s, V);
   } else {
-    staple_add<R, 2, 0, NC>(ch, eo, o, s, V);
-    staple_add<R, 2, 1, NC>(ch, eo, o, s, V);
+    staple_add<R, 2, 0, NC, ONE>(ch, eo, o, s, V);
+    staple_add<R, 2, 1, NC, ONE>(ch, eo, o, s, V);
   }
   return V;
 }
 
 // f/a_force.f:54-110: F = sum_mu [U(x)(iA(x+mu))U(x)^+ + U(x-mu)^+(iA(x-mu))U(x-mu)],
 // components F3 = Im(.)_a, F2 = Re(.)_b, F1 = Im(.)_b
-template <typename R, int MU, bool NC>
+template <typename R, int MU, bool NC, int ONE>
 __device__ __forceinline__ void force_add(const ChainDev& ch, int eo, const NbrOff& o, int s, R& f1, R& f2,
                                           R& f3) {
   const int oe = 1 - eo, nh = ch.nh;
   const R* A = reinterpret_cast<const R*>(ch.a);
   const int xp = s + o.p[MU], xm = s + o.m[MU];
-  su2<R> ux = ldU<R, NC>(ch, MU, eo, s);
-  su2<R> ud = ldU<R, NC>(ch, MU, oe, xm);
+  su2<R> ux = ldU<R, NC, ONE>(ch, MU, eo, s);
+  su2<R> ud = ldU<R, NC, ONE>(ch, MU, oe, xm);
   su2<R> t1 = nn(ux, ad(ldA<R, NC>(A, nh, oe, 0, xp), ldA<R, NC>(A, nh, oe, 1, xp), ldA<R, NC>(A, nh, oe, 2, xp), ux));
   su2<R> tb = dn(ud, an(ldA<R, NC>(A, nh, oe, 0, xm), ldA<R, NC>(A, nh, oe, 1, xm), ldA<R, NC>(A, nh, oe, 2, xm), ud));
   f3 = f3 + (t1.a.im + tb.a.im);
@@ -117,13 +175,13 @@ __device__ __forceinline__ void force_add(const ChainDev& ch, int eo, const NbrO
   f1 = f1 + (t1.b.im + tb.b.im);
 }
 
-template <typename R, bool NC = true>
+template <typename R, bool NC = true, int ONE = kTable>
 __device__ __forceinline__ void higgs_force(const ChainDev& ch, int eo, const NbrOff& o, int s, R& f1, R& f2,
                                             R& f3) {
   f1 = f2 = f3 = (R)0;
-  force_add<R, 0, NC>(ch, eo, o, s, f1, f2, f3);
-  force_add<R, 1, NC>(ch, eo, o, s, f1, f2, f3);
-  force_add<R, 2, NC>(ch, eo, o, s, f1, f2, f3);
+  force_add<R, 0, NC, ONE>(ch, eo, o, s, f1, f2, f3);
+  force_add<R, 1, NC, ONE>(ch, eo, o, s, f1, f2, f3);
+  force_add<R, 2, NC, ONE>(ch, eo, o, s, f1, f2, f3);
 }
 
 // Set up the uniform source of this pass (of hit `hit` of a multi-hit pass:
@@ -150,14 +208,16 @@ __device__ __forceinline__ bool setup_uniforms(const PassArgs& p, const ChainDev
 // One tile (BS * SPT consecutive sites of one chain, BS threads) of a Higgs
 // pass.  PDL: trigger dependents and wait for the previous kernel (per-pass
 // form only).
-template <typename R, int MODE, bool PDL, int SPT = 1, int BS = kBlock>
-__device__ __forceinline__ void higgs_tile(const PassArgs& p, int tile) {
+template <typename R, int MODE, bool PDL, int SPT = 1, int BS = kBlock, int ONE = kTable>
+__device__ __forceinline__ void higgs_tile(const Args<ONE>& p, int tile) {
   if (PDL && !p.trigger_late) pdl_trigger();
   // the chain table is written once at context creation: safe before pdl_wait
-  const int c = p.nchains > 1 ? find_chain(p.blk_begin, p.nchains, tile) : 0;
-  const ChainDev& ch = p.chains[c];
+  int ctile = tile;
+  const int c = find_tile(p, ctile);
+  const ChainDev& ch = chain_of(p, c);
+  const Cpl<R, ONE> cpl(p, ch);
   // a tile is BS * SPT consecutive sites; thread t takes t, t + BS, ...
-  const int s0 = p.s_lo + (tile - __ldg(p.blk_begin + c)) * BS * SPT + threadIdx.x;
+  const int s0 = p.s_lo + ctile * BS * SPT + threadIdx.x;
   const int eo = p.eo, nh = ch.nh, s_hi = nh - p.s_lo;
   const Coord X0 = site_coord(eo, s0 < s_hi ? s0 : p.s_lo, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
   unsigned acc[1] = {0u};
@@ -181,12 +241,15 @@ __device__ __forceinline__ void higgs_tile(const PassArgs& p, int tile) {
     Uniforms<R, NS> Un = Un0;
     if (r == 0 && early ? ok0 : setup_uniforms<R, NS>(p, ch, s, layout, Un)) {
       R f[3];
-      higgs_force<R, PDL>(ch, eo, no, s, f[0], f[1], f[2]);
+      higgs_force<R, PDL, ONE>(ch, eo, no, s, f[0], f[1], f[2]);
       R* A = reinterpret_cast<R*>(ch.a);
       R ao[3], an_[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) ao[k] = PDL ? A[((size_t)(eo * 3 + k)) * nh + s] : __ldcg(A + ((size_t)(eo * 3 + k)) * nh + s);
-      const R beta_a = (R)ch.beta_a, beta_2 = (R)ch.beta_2, beta_4 = (R)ch.beta_4;
+      for (int k = 0; k < 3; ++k) {
+        if (PDL) ao[k] = ONE ? (A + (size_t)(eo * 3 + k) * nh)[s] : A[((size_t)(eo * 3 + k)) * nh + s];
+        else ao[k] = __ldcg(A + ((size_t)(eo * 3 + k)) * nh + s);
+      }
+      const R beta_a = cpl.beta_a(), beta_2 = cpl.beta_2(), beta_4 = cpl.beta_4();
       R alph = (R)0, sf_o = (R)0, sf_n = (R)0;
       if constexpr (MODE == 0 || MODE == 1) {
         // f/ahiggs2.f:52-77 width / cxval / alph
@@ -201,8 +264,8 @@ __device__ __forceinline__ void higgs_tile(const PassArgs& p, int tile) {
           rr = M<R>::div((R)1, width);
           cxval = M<R>::div(M<R>::div((R)1, (R)2), width);
         } else {
-          rr = (R)ch.inv_beta2;      // 1/width, width = beta_2
-          cxval = (R)ch.cxval0;      // 1/beta_2/2
+          rr = cpl.inv_beta2();      // 1/width, width = beta_2
+          cxval = cpl.cxval0();      // 1/beta_2/2
         }
         if constexpr (MODE == 0) {
           // f/gauss.f:17-29: X = sqrt(-ln(W1)/R) cos(2 pi W2); f/ahiggs2.f:83-91
@@ -246,7 +309,8 @@ __device__ __forceinline__ void higgs_tile(const PassArgs& p, int tile) {
       if (boltz >= Un.v[acc_slot]) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          A[((size_t)(eo * 3 + k)) * nh + s] = an_[k];
+          if (ONE) (A + (size_t)(eo * 3 + k) * nh)[s] = an_[k];
+          else A[((size_t)(eo * 3 + k)) * nh + s] = an_[k];
           ao[k] = an_[k];
         }
         rho_o = rho_n;
@@ -270,13 +334,15 @@ __device__ __forceinline__ void higgs_tile(const PassArgs& p, int tile) {
 // NHIT = 3 is f/agauge1.f: the staple is built once and the heatbath +
 // Metropolis hit is repeated on the updated link, each hit with its own
 // uniforms (f/agauge1.f:95-198).
-template <typename R, int MU, int OR, bool PDL, int NHIT = 1, int SPT = 1, int BS = kBlock>
-__device__ __forceinline__ void link_tile(const PassArgs& p, int tile) {
+template <typename R, int MU, int OR, bool PDL, int NHIT = 1, int SPT = 1, int BS = kBlock, int ONE = kTable>
+__device__ __forceinline__ void link_tile(const Args<ONE>& p, int tile) {
   if (PDL && !p.trigger_late) pdl_trigger();
-  const int c = p.nchains > 1 ? find_chain(p.blk_begin, p.nchains, tile) : 0;
-  const ChainDev& ch = p.chains[c];
+  int ctile = tile;
+  const int c = find_tile(p, ctile);
+  const ChainDev& ch = chain_of(p, c);
+  const Cpl<R, ONE> cpl(p, ch);
   // a tile is BS * SPT consecutive sites; thread t takes t, t + BS, ...
-  const int s0 = p.s_lo + (tile - __ldg(p.blk_begin + c)) * BS * SPT + threadIdx.x;
+  const int s0 = p.s_lo + ctile * BS * SPT + threadIdx.x;
   const int eo = p.eo, oe = 1 - eo, nh = ch.nh, s_hi = nh - p.s_lo;
   const Coord X0 = site_coord(eo, s0 < s_hi ? s0 : p.s_lo, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
   unsigned cnt[2] = {0u, 0u};
@@ -298,9 +364,8 @@ __device__ __forceinline__ void link_tile(const PassArgs& p, int tile) {
     const NbrOff no = nbr_offsets(ch, X);
     Uniforms<R, OR ? 1 : 7> Un = Un0;
     if (r == 0 && early ? ok0 : setup_uniforms<R, OR ? 1 : 7>(p, ch, s, OR ? kPlanar : kTriple, Un)) {
-      const su2<R> V = staple<R, MU, PDL>(ch, eo, no, s);
-      const size_t li = ((size_t)(MU * 2 + eo)) * nh + s;
-      su2<R> uo = PDL ? LinkIO<R>::ld(ch.u, li) : LinkIO<R>::ld_cg(ch.u, li);
+      const su2<R> V = staple<R, MU, PDL, ONE>(ch, eo, no, s);
+      su2<R> uo = ldU<R, PDL, ONE>(ch, MU, eo, s);
       // f/agauge.f:71-84: normalised staple, 1/(beta |V|), 1/2 Re Tr(U Vhat)
       const R tn = M<R>::rsqrt(norm2(V));
       const su2<R> vh{{tn * V.a.re, tn * V.a.im}, {tn * V.b.re, tn * V.b.im}};
@@ -309,14 +374,14 @@ __device__ __forceinline__ void link_tile(const PassArgs& p, int tile) {
       const int xp = s + no.p[MU];
       const R x1 = ldA<R, PDL>(A, nh, eo, 0, s), x2 = ldA<R, PDL>(A, nh, eo, 1, s), x3 = ldA<R, PDL>(A, nh, eo, 2, s);
       const R y1 = ldA<R, PDL>(A, nh, oe, 0, xp), y2 = ldA<R, PDL>(A, nh, oe, 1, xp), y3 = ldA<R, PDL>(A, nh, oe, 2, xp);
-      const R beta_a = (R)ch.beta_a;
+      const R beta_a = cpl.beta_a();
       bool changed = false;
 #pragma unroll 1
       for (int hit = 0; hit < NHIT; ++hit) {
         if (hit > 0 && !setup_uniforms<R, OR ? 1 : 7>(p, ch, s, OR ? kPlanar : kTriple, Un, hit)) break;
         su2<R> hn;
         if constexpr (!OR) {
-          const R t1 = M<R>::div(tn, (R)ch.beta);
+          const R t1 = M<R>::div(tn, cpl.beta());
           const R t2 = (uo.a * vh.a - uo.b * cj(vh.b)).re;
           // f/heat_kpi.f:33-98 single-trial Kennedy-Pendleton
           R a1 = Un.v[0], a2 = Un.v[1], a3 = Un.v[2];
@@ -352,7 +417,11 @@ __device__ __forceinline__ void link_tile(const PassArgs& p, int tile) {
           cnt[OR ? 0 : 1] += 1u;
         }
       }
-      if (changed) LinkIO<R>::st(ch.u, li, p.fuse_renorm ? unitarise64(uo) : uo);
+      if (changed) {
+        const su2<R> un = p.fuse_renorm ? unitarise64(uo) : uo;
+        if (ONE) LinkIO<R>::st(static_cast<char*>(ch.u) + (size_t)(MU * 2 + eo) * nh * LinkIO<R>::kBytes, s, un);
+        else LinkIO<R>::st(ch.u, (size_t)(MU * 2 + eo) * nh + s, un);
+      }
       // f/agauge.f:179-185 plaquette against the staple
       if (!OR && p.part) pl[0] += (double)nn(uo, V).a.re;
     }
@@ -477,23 +546,34 @@ constexpr int min_blocks_bs() {
   return OCC ? OCC / BS : (min_blocks<R>() * kBlock / BS > 0 ? min_blocks<R>() * kBlock / BS : 1);
 }
 
-template <typename R, int MODE, int SPT, int BS, int OCC = 0>
-__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) higgs_kernel(PassArgs p) {
+// ONE, where a kernel finds its chain.  kOne: a single-chain context's chain
+// in the parameter bank: its extents, plane addresses and couplings are
+// uniform and need no loads, conversions or registers of their own.  Sweeps
+// without measurements, the same tile: 16^3 22.1 -> 20.4 us, 64^3 38.6 ->
+// 36.6, with 4 overrelaxations 125.0 -> 115.8, 128^3 301 -> 290, FP64 64^3
+// 93.8 -> 88.8.  kMany: a batch's table in the parameter bank, found by the
+// block's tile: 96 chains of 16^3-48^3 with two sites per thread 796 -> 762
+// us, one 836 -> 818.  kTable: the table in memory (kParamTiles).  The passes
+// of 64^3 and above are bound by instruction issue (a link heatbath takes
+// ~700 warp instructions per site, 335 of them FP32 arithmetic, ~70% of the
+// issue slots of an active SM).
+template <typename R, int MODE, int SPT, int BS, int OCC, int ONE>
+__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) higgs_kernel(Args<ONE> p) {
   if (kReduceBehind<SPT> && p.rb_nitems && (int)blockIdx.x >= p.ntiles) reduce_behind(p);
-  else higgs_tile<R, MODE, true, SPT, BS>(p, blockIdx.x);
+  else higgs_tile<R, MODE, true, SPT, BS, ONE>(p, blockIdx.x);
 }
 
-template <typename R, int MU, int OR, int SPT, int BS, int OCC = 0>
-__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) link_kernel(PassArgs p) {
+template <typename R, int MU, int OR, int SPT, int BS, int OCC, int ONE>
+__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) link_kernel(Args<ONE> p) {
   if (kReduceBehind<SPT> && p.rb_nitems && (int)blockIdx.x >= p.ntiles) reduce_behind(p);
-  else link_tile<R, MU, OR, true, 1, SPT, BS>(p, blockIdx.x);
+  else link_tile<R, MU, OR, true, 1, SPT, BS, ONE>(p, blockIdx.x);
 }
 
 // f/agauge1.f (3 hits)
-template <typename R, int MU, int SPT, int BS, int OCC = 0>
-__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) link3_kernel(PassArgs p) {
+template <typename R, int MU, int SPT, int BS, int OCC, int ONE>
+__global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) link3_kernel(Args<ONE> p) {
   if (kReduceBehind<SPT> && p.rb_nitems && (int)blockIdx.x >= p.ntiles) reduce_behind(p);
-  else link_tile<R, MU, 0, true, 3, SPT, BS>(p, blockIdx.x);
+  else link_tile<R, MU, 0, true, 3, SPT, BS, ONE>(p, blockIdx.x);
 }
 
 // level 2, item w = (chain c, slot i); nothing to do for a one-chunk chain
@@ -767,14 +847,14 @@ __global__ void __launch_bounds__(kFinSmallWarps * 32) finalize_small_kernel(Fin
 // runs beside this pass's tiles instead of between the sweeps.
 template <typename R, int BS>
 __global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, 0>())
-    higgs_fin_kernel(PassArgs p, const __grid_constant__ FinalizeArgs fp) {
+    higgs_fin_kernel(PassArgsOne p, const __grid_constant__ FinalizeArgs fp) {
   if ((int)blockIdx.x >= p.ntiles) {
     __shared__ SmallFinSmem S;
     pdl_wait();
     pdl_trigger();
     finalize_small_body<true>(fp, S);
   } else {
-    higgs_tile<R, 0, true, 1, BS>(p, blockIdx.x);
+    higgs_tile<R, 0, true, 1, BS, kOne>(p, blockIdx.x);
   }
 }
 
@@ -960,26 +1040,52 @@ __global__ void debug_force_kernel(const ChainDev* chp, int eo, double* out) {
 // ------------------------------------------------------------------ launchers
 // The pass kernels and the finalize kernel are launched with programmatic
 // dependent launch (lce_common.cuh: launch_pdl / pdl_wait).
-template <typename R, int SPT, int BS, int OCC = 0>
-void launch_higgs_t(int mode, const PassArgs& a, int nblocks, cudaStream_t s) {
-  void (*k)(PassArgs) = mode == 0 ? higgs_kernel<R, 0, SPT, BS, OCC>
-                                  : (mode == 1 ? higgs_kernel<R, 1, SPT, BS, OCC> : higgs_kernel<R, 2, SPT, BS, OCC>);
-  (void)launch_pdl(k, nblocks, BS, 0, s, a);
+// the single-chain kernels' arguments: the batch's first chain
+PassArgsOne one_of(const PassArgsMany& a) {
+  PassArgsOne o;
+  static_cast<PassArgs&>(o) = a;
+  const ChainDev& d = o.one = a.ch[0];
+  o.beta = (float)d.beta;
+  o.beta_a = (float)d.beta_a;
+  o.beta_2 = (float)d.beta_2;
+  o.beta_4 = (float)d.beta_4;
+  o.inv_beta2 = (float)d.inv_beta2;
+  o.cxval0 = (float)d.cxval0;
+  return o;
 }
 
-template <typename R, int SPT, int BS, int OCC = 0>
-void launch_link_t(int mode, int mu, const PassArgs& a, int nblocks, cudaStream_t s) {
-  void (*k)(PassArgs);
-  if (mode == 0)
-    k = mu == 0 ? link_kernel<R, 0, 0, SPT, BS, OCC>
-                : (mu == 1 ? link_kernel<R, 1, 0, SPT, BS, OCC> : link_kernel<R, 2, 0, SPT, BS, OCC>);
-  else if (mode == 1)
-    k = mu == 0 ? link_kernel<R, 0, 1, SPT, BS, OCC>
-                : (mu == 1 ? link_kernel<R, 1, 1, SPT, BS, OCC> : link_kernel<R, 2, 1, SPT, BS, OCC>);
-  else
-    k = mu == 0 ? link3_kernel<R, 0, SPT, BS, OCC>
-                : (mu == 1 ? link3_kernel<R, 1, SPT, BS, OCC> : link3_kernel<R, 2, SPT, BS, OCC>);
+template <typename R, int SPT, int BS, int OCC, int ONE>
+void launch_higgs_k(int mode, const Args<ONE>& a, int nblocks, cudaStream_t s) {
+  void (*k)(Args<ONE>) = mode == 0 ? higgs_kernel<R, 0, SPT, BS, OCC, ONE>
+                                  : (mode == 1 ? higgs_kernel<R, 1, SPT, BS, OCC, ONE> : higgs_kernel<R, 2, SPT, BS, OCC, ONE>);
   (void)launch_pdl(k, nblocks, BS, 0, s, a);
+}
+template <typename R, int SPT, int BS, int OCC = 0>
+void launch_higgs_t(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) {
+  if (a.nchains == 1) launch_higgs_k<R, SPT, BS, OCC, kOne>(mode, one_of(a), nblocks, s);
+  else if (a.many) launch_higgs_k<R, SPT, BS, OCC, kMany>(mode, a, nblocks, s);
+  else launch_higgs_k<R, SPT, BS, OCC, kTable>(mode, a, nblocks, s);
+}
+
+template <typename R, int SPT, int BS, int OCC, int ONE>
+void launch_link_k(int mode, int mu, const Args<ONE>& a, int nblocks, cudaStream_t s) {
+  void (*k)(Args<ONE>);
+  if (mode == 0)
+    k = mu == 0 ? link_kernel<R, 0, 0, SPT, BS, OCC, ONE>
+                : (mu == 1 ? link_kernel<R, 1, 0, SPT, BS, OCC, ONE> : link_kernel<R, 2, 0, SPT, BS, OCC, ONE>);
+  else if (mode == 1)
+    k = mu == 0 ? link_kernel<R, 0, 1, SPT, BS, OCC, ONE>
+                : (mu == 1 ? link_kernel<R, 1, 1, SPT, BS, OCC, ONE> : link_kernel<R, 2, 1, SPT, BS, OCC, ONE>);
+  else
+    k = mu == 0 ? link3_kernel<R, 0, SPT, BS, OCC, ONE>
+                : (mu == 1 ? link3_kernel<R, 1, SPT, BS, OCC, ONE> : link3_kernel<R, 2, SPT, BS, OCC, ONE>);
+  (void)launch_pdl(k, nblocks, BS, 0, s, a);
+}
+template <typename R, int SPT, int BS, int OCC = 0>
+void launch_link_t(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStream_t s) {
+  if (a.nchains == 1) launch_link_k<R, SPT, BS, OCC, kOne>(mode, mu, one_of(a), nblocks, s);
+  else if (a.many) launch_link_k<R, SPT, BS, OCC, kMany>(mode, mu, a, nblocks, s);
+  else launch_link_k<R, SPT, BS, OCC, kTable>(mode, mu, a, nblocks, s);
 }
 
 // Tile shapes compiled: FP32 (BS, SPT) in {128, 256, 512} x {1} and
@@ -987,7 +1093,7 @@ void launch_link_t(int mode, int mu, const PassArgs& a, int nblocks, cudaStream_
 // registers), and (128, 1) at 56 registers (a.occ = 1152); the FP64
 // validation path only BS = 256.
 template <typename R>
-void launch_higgs(int mode, const PassArgs& a, int nblocks, cudaStream_t s) {
+void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
     if (a.bs == 128 && a.occ == 1152) {
       launch_higgs_t<R, 1, 128, 1152>(mode, a, nblocks, s);
@@ -1012,7 +1118,7 @@ void launch_higgs(int mode, const PassArgs& a, int nblocks, cudaStream_t s) {
 }
 
 template <typename R>
-void launch_link(int mode, int mu, const PassArgs& a, int nblocks, cudaStream_t s) {
+void launch_link(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
     if (a.bs == 128 && a.occ == 1152) {
       launch_link_t<R, 1, 128, 1152>(mode, mu, a, nblocks, s);
@@ -1039,25 +1145,25 @@ void launch_link(int mode, int mu, const PassArgs& a, int nblocks, cudaStream_t 
 // the first pass of a sweep carrying the previous sweep's finalize (one site
 // per thread, 128 (64 registers), 256, 448 or 512 threads in FP32; 256 in FP64)
 template <typename R>
-void launch_higgs_fin(const PassArgs& a, const FinalizeArgs& fp, int nblocks, cudaStream_t s) {
+void launch_higgs_fin(const PassArgsMany& a, const FinalizeArgs& fp, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
     if (a.bs == 128) {
-      (void)launch_pdl(higgs_fin_kernel<R, 128>, nblocks, 128, 0, s, a, fp);
+      (void)launch_pdl(higgs_fin_kernel<R, 128>, nblocks, 128, 0, s, one_of(a), fp);
       return;
     }
     if (a.bs == 448) {
-      (void)launch_pdl(higgs_fin_kernel<R, 448>, nblocks, 448, 0, s, a, fp);
+      (void)launch_pdl(higgs_fin_kernel<R, 448>, nblocks, 448, 0, s, one_of(a), fp);
       return;
     }
     if (a.bs == 512) {
-      (void)launch_pdl(higgs_fin_kernel<R, 512>, nblocks, 512, 0, s, a, fp);
+      (void)launch_pdl(higgs_fin_kernel<R, 512>, nblocks, 512, 0, s, one_of(a), fp);
       return;
     }
   }
-  (void)launch_pdl(higgs_fin_kernel<R, 256>, nblocks, 256, 0, s, a, fp);
+  (void)launch_pdl(higgs_fin_kernel<R, 256>, nblocks, 256, 0, s, one_of(a), fp);
 }
-template void launch_higgs_fin<float>(const PassArgs&, const FinalizeArgs&, int, cudaStream_t);
-template void launch_higgs_fin<double>(const PassArgs&, const FinalizeArgs&, int, cudaStream_t);
+template void launch_higgs_fin<float>(const PassArgsMany&, const FinalizeArgs&, int, cudaStream_t);
+template void launch_higgs_fin<double>(const PassArgsMany&, const FinalizeArgs&, int, cudaStream_t);
 
 void launch_finalize(const FinalizeArgs& f, cudaStream_t s) {
   if (f.nchains == 1 && f.nchunks <= kSmallChunks) {
@@ -1116,8 +1222,8 @@ void launch_debug_force(const ChainDev* ch, int eo, double* out, int nh, cudaStr
 }
 
 #define LCE_INST(R)                                                                          \
-  template void launch_higgs<R>(int, const PassArgs&, int, cudaStream_t);                  \
-  template void launch_link<R>(int, int, const PassArgs&, int, cudaStream_t);              \
+  template void launch_higgs<R>(int, const PassArgsMany&, int, cudaStream_t);                  \
+  template void launch_link<R>(int, int, const PassArgsMany&, int, cudaStream_t);              \
   template int persistent_grid<R>();                                                         \
   template cudaError_t launch_persistent<R>(const PersistArgs&, int, cudaStream_t);          \
   template void launch_renorm<R>(void*, size_t, cudaStream_t);                             \
