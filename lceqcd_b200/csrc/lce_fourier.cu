@@ -53,9 +53,10 @@
 // X = -i s.sigma: with Y = X(x+mu),
 //   F'(0)  = sum c_mu Re a[X U - U Y]
 //   F''(0) = sum c_mu Re a[X^2 U + U Y^2 - 2 X U Y],
-// alpha = F'(0) / -F''(0) (exact per link to second order).  Four more
-// kernels per iteration: the beta reduction, the line derivatives, the alpha
-// reduction and g = exp(alpha X) per site.  The step is bounded by a trust
+// alpha = F'(0) / -F''(0) (exact per link to second order).  Three
+// more kernels per iteration: the beta reduction, the line derivatives and the
+// alpha reduction; g = exp(alpha X) is formed by the kernel that applies it
+// (on z-slabs by a kernel of its own).  The step is bounded by a trust
 // region (fa_alpha_kernel).
 #include <algorithm>
 #include <cstring>
@@ -106,10 +107,14 @@ struct FaLines {
   // line stride: a line in natural order, or (between the two steps) N1 rows
   // of N2 points, each row padded by one; n + N1 + 1 = 2 mod 32 words apart
   static constexpr int ld = N2 > 1 ? N1 * (N2 + 1) + 1 : n + 1;
+  // the line stride where columns, not lines, go to consecutive threads
+  // (fa_g_kernel): N2 mod 16 float2, so that a half-warp's 16 / N2 lines do
+  // not meet in a bank
+  static constexpr int ldx = N1 * (N2 + 1) + (N2 < 16 ? N2 : 1);
   static constexpr int ntw = n / 2 > 0 ? n / 2 : 1;              // twiddle table entries
   // lines, ntab twiddle tables and nd doubles
-  static constexpr size_t smem(int ntab, int nd) {
-    return ((size_t)NLT * ld + (size_t)ntab * ntw) * sizeof(FftC) + (size_t)nd * sizeof(double);
+  static constexpr size_t smem(int ntab, int nd, int stride = ld) {
+    return ((size_t)NLT * stride + (size_t)ntab * ntw) * sizeof(FftC) + (size_t)nd * sizeof(double);
   }
 };
 
@@ -238,6 +243,42 @@ __device__ __forceinline__ void fft2_lines(FftC* d, const FftC* tw) {
   __syncthreads();
 }
 
+// The two steps of fft2_lines on their own, for the kernels that read the
+// first step's points from global memory or write the second step's there
+// (lines of 32 to 512 points; the same arithmetic, so the same bits): the
+// block's points pass through shared memory once per transform, between the
+// steps, instead of three times.
+template <int LOGN>
+constexpr bool kFaDirect = LOGN >= 5 && LOGN <= 9;
+
+// step 1 of column n2: N1 points of stride N2 -> DFT, twiddles
+template <int LOGN>
+__device__ __forceinline__ void fft_step1(FftC (&r)[FaLines<LOGN>::N1], int n2, const FftC* tw) {
+  using G = FaLines<LOGN>;
+  dft_reg<G::N1, G::n>(r, tw);
+#pragma unroll
+  for (int k1 = 1; k1 < G::N1; ++k1) {
+    const int e = n2 * k1;  // < n; W_n^e = -W_n^(e - n/2) for e >= n/2
+    const FftC w = e < G::n / 2 ? tw[e] : FftC{-tw[e - G::n / 2].x, -tw[e - G::n / 2].y};
+    r[k1] = cmul(w, r[k1]);
+  }
+}
+// row k1 of a line at `line`: stored by step 1 as column n2, read by step 2
+template <int LOGN>
+__device__ __forceinline__ void fft_put_column(FftC* line, int n2, const FftC (&r)[FaLines<LOGN>::N1]) {
+  using G = FaLines<LOGN>;
+#pragma unroll
+  for (int k1 = 0; k1 < G::N1; ++k1) line[k1 * (G::N2 + 1) + n2] = r[k1];
+}
+// step 2 of row k1: X[k1 + N1 k2] in w[k2]
+template <int LOGN>
+__device__ __forceinline__ void fft_step2(const FftC* line, int k1, FftC (&w)[FaLines<LOGN>::N2], const FftC* tw) {
+  using G = FaLines<LOGN>;
+#pragma unroll
+  for (int i = 0; i < G::N2; ++i) w[i] = line[k1 * (G::N2 + 1) + i];
+  dft_reg<G::N2, G::n>(w, tw);
+}
+
 template <typename R>
 __device__ __forceinline__ su2<double> to_d(su2<R> u) {
   return su2<double>{{(double)u.a.re, (double)u.a.im}, {(double)u.b.re, (double)u.b.im}};
@@ -295,6 +336,44 @@ __device__ __forceinline__ size_t nat_index(const FaArgs& a, int l, int k) {
   return ((((size_t)k << s2) + (l >> s1)) << s1) + (l & m1);                          // l = x + L1 y
 }
 
+// The records of the scalar kernels (check, beta, alpha): thread t adds the
+// records t, t + 1024, ... in order, eight in flight.  (One block; done by the
+// last block of the kernel before, the fence and the ticket of its thousands
+// of blocks cost more than the launch: 128^3 line kernel 32 -> 53 us.)
+template <int NQ>
+__device__ __forceinline__ void fa_sums(const double* part, int n, double* t) {
+  double v[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+#pragma unroll 8
+  for (int b = threadIdx.x; b < n; b += 1024) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] += part[(size_t)b * NQ + q];
+  }
+  block_reduce_store<NQ>(v, t);
+  __syncthreads();
+}
+
+// (2) theta = sum / nh (odd sites); count; done flag at theta <= gf_limit or
+// the cap
+__global__ void __launch_bounds__(1024) fa_check_kernel(const ChainDev* chp, ChainState* cst, const double* part,
+                                                        int nblocks, int adapt) {
+  if (cst->gf_done) return;
+  __shared__ double tot[1];
+  fa_sums<1>(part, nblocks, tot);
+  if (threadIdx.x == 0) {
+    const double theta = tot[0] / chp->nh;
+    const int it = cst->gf_iters + 1;
+    // a step that doubled theta overshot (far from the Landau gauge the
+    // linearised step can be too long): shorten it for the rest of the run
+    // (the conjugate-gradient form chooses its own step)
+    if (adapt && it > 1 && theta > 2.0 * cst->gf_theta) cst->gf_step = fmax(0.1, 0.7 * cst->gf_step);
+    cst->gf_iters = it;
+    cst->gf_theta = theta;
+    if (!(theta > cst->gf_limit) || (cst->gf_cap > 0 && it >= cst->gf_cap)) cst->gf_done = 1;
+  }
+}
+
 // (1) Delta on x-lines, forward FFT along x; partials of theta.  A block
 // takes NL x-lines of both fields: lines 0 .. NL-1 hold Delta_b, NL .. 2NL-1
 // hold Delta_a3.
@@ -312,7 +391,7 @@ __global__ void __launch_bounds__(kFaThreads) fa_div_kernel(FaArgs a) {
   load_twiddles(tw, a.tw, n, -1);
   const double al = ch.alpha;
   double q[1] = {0.0};
-  for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
+  for (int e = threadIdx.x; e < NL * n; e += kFaThreads) {
     const int j = e >> LOGN, x = e & (n - 1), l = l0 + j;
     FftC v0{0, 0}, v1{0, 0};
     if (l < nlines) {
@@ -328,8 +407,8 @@ __global__ void __launch_bounds__(kFaThreads) fa_div_kernel(FaArgs a) {
 #pragma unroll
       for (int mu = 0; mu < 3; ++mu) {
         const double c = mu == 2 ? al : 1.0;
-        const su2<R> u = LinkIO<R>::ld_cg(ch.uf, ((size_t)(mu * 2 + p)) * ch.nh + s);
-        const su2<R> w = LinkIO<R>::ld_cg(ch.uf, ((size_t)(mu * 2 + op)) * ch.nh + xm[mu]);
+        const su2<R> u = LinkIO<R>::ld(ch.uf, ((size_t)(mu * 2 + p)) * ch.nh + s);
+        const su2<R> w = LinkIO<R>::ld(ch.uf, ((size_t)(mu * 2 + op)) * ch.nh + xm[mu]);
         d3 += c * ((double)u.a.im - (double)w.a.im);
         dbr += c * ((double)u.b.re - (double)w.b.re);
         dbi += c * ((double)u.b.im - (double)w.b.im);
@@ -343,10 +422,37 @@ __global__ void __launch_bounds__(kFaThreads) fa_div_kernel(FaArgs a) {
   }
   block_reduce_store<1>(q, a.part + blockIdx.x);
   __syncthreads();
-  fft2_lines<LOGN>(d, tw);
   const size_t V = (size_t)a.L[0] * a.L[1] * a.L[2];
   FftC* F = reinterpret_cast<FftC*>(a.fft);
   const int lg0 = a.zg0 * a.L[1];  // the whole lattice's line of local line 0
+  if constexpr (kFaDirect<LOGN>) {
+    // step 1 from shared memory, lines to consecutive threads; step 2 to
+    // global memory, rows to consecutive threads (runs of N1 points)
+    constexpr int N1 = G::N1, N2 = G::N2, NLT = G::NLT;
+    static_assert(NLT * N2 <= kFaThreads, "one column per thread");
+    FftC r[N1];
+    const int j1 = threadIdx.x % NLT, n2 = threadIdx.x / NLT;
+    if (n2 < N2) {
+#pragma unroll
+      for (int i = 0; i < N1; ++i) r[i] = d[j1 * ld + i * N2 + n2];
+      fft_step1<LOGN>(r, n2, tw);
+    }
+    __syncthreads();
+    if (n2 < N2) fft_put_column<LOGN>(d + j1 * ld, n2, r);
+    __syncthreads();
+#pragma unroll
+    for (int q2 = 0; q2 < NLT * N1 / kFaThreads; ++q2) {
+      const int it = threadIdx.x + q2 * kFaThreads, k1 = it % N1, j = it / N1, l = l0 + (j & (NL - 1));
+      FftC w[N2];
+      fft_step2<LOGN>(d + j * ld, k1, w, tw);
+      if (l >= nlines) continue;
+      FftC* Fl = F + (j >= NL ? V : 0) + nat_index<0>(a, lg0 + l, k1);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) Fl[k2 * N1] = w[k2];
+    }
+    return;
+  }
+  fft2_lines<LOGN>(d, tw);
   for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
     const int j = e >> LOGN, k = e & (n - 1), l = l0 + j;
     if (l >= nlines) continue;
@@ -356,26 +462,126 @@ __global__ void __launch_bounds__(kFaThreads) fa_div_kernel(FaArgs a) {
   }
 }
 
-// (2) theta = sum / nh (odd sites); count; done flag at theta <= gf_limit or
-// the cap
-__global__ void __launch_bounds__(1024) fa_check_kernel(const ChainDev* chp, ChainState* cst, const double* part,
-                                                        int nblocks, int adapt) {
-  if (cst->gf_done) return;
-  double v[1] = {0.0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v[0] += part[b];
-  __shared__ double tot[1];
-  block_reduce_store<1>(v, tot);
+// The transformed lines at d scaled by gamma / (p_c^2 V), element e -> (line j
+// = e % NL, position k = e / NL).  CG: also the block's sums and F kept as the
+// next F_prev, in two buffers: a read-modify-write of one stalled every
+// element on its own load (5x the kernel's time at 128^3).  The sums take the
+// weight 1/(4 p^2) = (1/p^2) / 4 (exact), the element is scaled by gamma /
+// (4 V p^2) = gv (1/p^2) -- one FP64 division per element.
+template <int AX, int LOGN, bool CG>
+__device__ __forceinline__ void fa_scale(const FaArgs& a, FftC* d, const double* sz2, const double* sxy, int l0,
+                                         int nlines) {
+  using G = FaLines<LOGN>;
+  constexpr int n = G::n, ld = G::ld, NL = G::NLT, LNL = kFaBlockLog - LOGN;
+  const size_t V = (size_t)a.L[0] * a.L[1] * a.L[2];
+  const double gv = (a.cst ? a.cst->gf_step : a.gamma) / (4.0 * (double)V);
+  if (CG) {
+    const int par = a.cg->parity;
+    FftC* Pn = reinterpret_cast<FftC*>(a.prev) + ((size_t)par * 2 + blockIdx.y) * V;
+    const FftC* Po = reinterpret_cast<const FftC*>(a.prev) + ((size_t)(par ^ 1) * 2 + blockIdx.y) * V;
+    double v[2] = {0.0, 0.0};
+    // four elements' loads of the previous F in flight together
+    constexpr int kBatch = 4;
+    static_assert(NL * n % (kBatch * kFaThreads) == 0, "whole batches");
+    for (int e0 = threadIdx.x; e0 < NL * n; e0 += kBatch * kFaThreads) {
+      FftC pv[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int e = e0 + b * kFaThreads, l = l0 + (e & (NL - 1));
+        if (l < nlines) pv[b] = __ldg(Po + nat_index<AX>(a, l, e >> LNL));
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int e = e0 + b * kFaThreads, j = e & (NL - 1), k = e >> LNL, l = l0 + j;
+        const int q = j * ld + k;
+        if (l >= nlines) continue;
+        const FftC f = d[q];
+        Pn[nat_index<AX>(a, l, k)] = f;
+        if ((l | k) == 0) {
+          d[q] = FftC{0, 0};
+          continue;
+        }
+        const double r = 1.0 / (sxy[j] + sz2[k]), m0 = 0.25 * r, m = gv * r;
+        v[0] += m0 * ((double)f.x * f.x + (double)f.y * f.y);
+        v[1] += m0 * ((double)f.x * pv[b].x + (double)f.y * pv[b].y);
+        d[q] = FftC{(FftR)(f.x * m), (FftR)(f.y * m)};
+      }
+    }
+    block_reduce_store<2>(v, a.cgpart + 2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x));
+  } else {
+    for (int e = threadIdx.x; e < NL * n; e += kFaThreads) {
+      const int j = e >> LOGN, kz = e & (n - 1), l = l0 + j;
+      const double p2 = sxy[j] + sz2[kz];
+      const double m = (l | kz) ? gv / p2 : 0.0;
+      const int q = j * ld + kz;
+      d[q] = FftC{(FftR)(d[q].x * m), (FftR)(d[q].y * m)};
+    }
+  }
+}
+
+// The body of fa_fft_kernel with the points read from and written to global
+// memory by the transform's steps.  Thread t takes line t % NL throughout
+// (consecutive lines are consecutive x): column t / NL in step 1, rows t / NL
+// + (256 / NL) q in step 2.  In the graph at 128^3 / 256^3: a y pass 18.3 -> 13.0
+// / 98 us (5.5 TB/s), the z transforms of the conjugate-gradient form 46.5 ->
+// 41.8 / 343 us (held by their FP64 divisions and five barriers per block).
+template <int AX, bool SCALE, int LOGN, bool CG>
+__device__ __forceinline__ void fft_direct(const FaArgs& a, FftC* d, const FftC* tw, const FftC* twi, const double* sz2,
+                                           const double* sxy, FftC* F, int l0, int nlines) {
+  using G = FaLines<LOGN>;
+  constexpr int N1 = G::N1, N2 = G::N2, NL = G::NLT, ld = G::ld, IB = NL * N1 / kFaThreads;
+  static_assert(NL * N2 <= kFaThreads && NL * N1 % kFaThreads == 0, "items per thread");
+  const int j = threadIdx.x % NL, t = threadIdx.x / NL, l = l0 + j;
+  const bool live = l < nlines;
+  FftC r[N1];
+  if (t < N2) {
+#pragma unroll
+    for (int i = 0; i < N1; ++i) r[i] = live ? F[nat_index<AX>(a, l, i * N2 + t)] : FftC{0, 0};
+  }
+  if (CG && live) {
+    // the previous F, needed by the scaling, into L2 meanwhile
+    const FftC* Po = reinterpret_cast<const FftC*>(a.prev) +
+                     ((size_t)(a.cg->parity ^ 1) * 2 + blockIdx.y) * ((size_t)a.L[0] * a.L[1] * a.L[2]);
+    for (int k = t; k < G::n; k += kFaThreads / NL)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(Po + nat_index<AX>(a, l, k)));
+  }
+  __syncthreads();  // the twiddles
+  FftC* line = d + j * ld;
+  if (t < N2) {
+    fft_step1<LOGN>(r, t, tw);
+    fft_put_column<LOGN>(line, t, r);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double theta = tot[0] / chp->nh;
-    const int it = cst->gf_iters + 1;
-    // a step that doubled theta overshot (far from the Landau gauge the
-    // linearised step can be too long): shorten it for the rest of the run
-    // (the conjugate-gradient form chooses its own step)
-    if (adapt && it > 1 && theta > 2.0 * cst->gf_theta) cst->gf_step = fmax(0.1, 0.7 * cst->gf_step);
-    cst->gf_iters = it;
-    cst->gf_theta = theta;
-    if (!(theta > cst->gf_limit) || (cst->gf_cap > 0 && it >= cst->gf_cap)) cst->gf_done = 1;
+  FftC w[IB][N2];
+#pragma unroll
+  for (int q = 0; q < IB; ++q) fft_step2<LOGN>(line, t + q * (kFaThreads / NL), w[q], tw);
+  if constexpr (SCALE) {
+    // the scaling (and the sums) from shared memory in natural order: with the
+    // elements in the step's registers the kernel spilled at 64 and at 80
+    __syncthreads();  // the rows have been read
+#pragma unroll
+    for (int q = 0; q < IB; ++q)
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) line[t + q * (kFaThreads / NL) + N1 * k2] = w[q][k2];
+    __syncthreads();
+    fa_scale<AX, LOGN, CG>(a, d, sz2, sxy, l0, nlines);
+    __syncthreads();
+    if (t < N2) {
+#pragma unroll
+      for (int i = 0; i < N1; ++i) r[i] = line[i * N2 + t];
+      fft_step1<LOGN>(r, t, twi);
+    }
+    __syncthreads();
+    if (t < N2) fft_put_column<LOGN>(line, t, r);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < IB; ++q) fft_step2<LOGN>(line, t + q * (kFaThreads / NL), w[q], twi);
+  }
+  if (live) {
+#pragma unroll
+    for (int q = 0; q < IB; ++q)
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) F[nat_index<AX>(a, l, t + q * (kFaThreads / NL) + N1 * k2)] = w[q][k2];
   }
 }
 
@@ -413,6 +619,10 @@ __global__ void __launch_bounds__(kFaThreads, LOGN <= 8 ? 4 : 1) fa_fft_kernel(F
       sxy[j] = sx * sx + sy * sy;
     }
   }
+  if constexpr (kFaDirect<LOGN>) {
+    fft_direct<AX, SCALE, LOGN, CG>(a, d, tw, twi, sz2, sxy, F, l0, nlines);
+    return;
+  }
   // element e -> (line j = e % NL, position k = e / NL): consecutive threads
   // read consecutive lines, i.e. consecutive x
   for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
@@ -421,44 +631,8 @@ __global__ void __launch_bounds__(kFaThreads, LOGN <= 8 ? 4 : 1) fa_fft_kernel(F
   }
   __syncthreads();
   fft2_lines<LOGN>(d, tw);
-  if (CG) {
-    // two buffers: a read-modify-write of one stalled every element on its
-    // own load (5x the kernel's time at 128^3).  One pass: the sums with the
-    // weight 1/(4 p^2) = (1/p^2) / 4 (exact), then the element scaled by
-    // gamma / (4 V p^2) = gv (1/p^2) -- one FP64 division per element
-    const int par = a.cg->parity;
-    FftC* Pn = reinterpret_cast<FftC*>(a.prev) + ((size_t)par * 2 + blockIdx.y) * V;
-    const FftC* Po = reinterpret_cast<const FftC*>(a.prev) + ((size_t)(par ^ 1) * 2 + blockIdx.y) * V;
-    const double gv = (a.cst ? a.cst->gf_step : a.gamma) / (4.0 * (double)V);
-    double v[2] = {0.0, 0.0};
-    for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
-      const int j = e & (NL - 1), k = e >> LNL, l = l0 + j;
-      const int q = j * ld + k;
-      if (l >= nlines) continue;
-      const size_t gi = nat_index<AX>(a, l, k);
-      const FftC f = d[q], pv = __ldg(Po + gi);
-      Pn[gi] = f;
-      if ((l | k) == 0) {
-        d[q] = FftC{0, 0};
-        continue;
-      }
-      const double r = 1.0 / (sxy[j] + sz2[k]), m0 = 0.25 * r, m = gv * r;
-      v[0] += m0 * ((double)f.x * f.x + (double)f.y * f.y);
-      v[1] += m0 * ((double)f.x * pv.x + (double)f.y * pv.y);
-      d[q] = FftC{(FftR)(f.x * m), (FftR)(f.y * m)};
-    }
-    block_reduce_store<2>(v, a.cgpart + 2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x));
-    __syncthreads();
-    fft2_lines<LOGN>(d, twi);
-  } else if (SCALE) {
-    const double gv = (a.cst ? a.cst->gf_step : a.gamma) / (4.0 * (double)V);
-    for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
-      const int j = e >> LOGN, kz = e & (n - 1), l = l0 + j;
-      const double p2 = sxy[j] + sz2[kz];
-      const double m = (l | kz) ? gv / p2 : 0.0;
-      const int q = j * ld + kz;
-      d[q] = FftC{(FftR)(d[q].x * m), (FftR)(d[q].y * m)};
-    }
+  if constexpr (SCALE) {
+    fa_scale<AX, LOGN, CG>(a, d, sz2, sxy, l0, nlines);
     __syncthreads();
     fft2_lines<LOGN>(d, twi);
   }
@@ -470,10 +644,29 @@ __global__ void __launch_bounds__(kFaThreads, LOGN <= 8 ? 4 : 1) fa_fft_kernel(F
 
 // (6) inverse FFT along x; g(x) = exp(-i omega.sigma) per site (CG: the
 // direction s = omega + beta s instead)
+// g(x) = exp(-i omega.sigma) of one site into gstep
+__device__ __forceinline__ void fa_site_g(const FaArgs& a, size_t gi, double w3, double wbr, double wbi) {
+  const double nw = sqrt(w3 * w3 + wbr * wbr + wbi * wbi);
+  su2<double> gg{{1.0, 0.0}, {0.0, 0.0}};
+  if (nw > 0.0) {
+    double sn, cs;
+    sincos(nw, &sn, &cs);
+    const double f = sn / nw;
+    gg = su2<double>{{cs, -f * w3}, {-f * wbr, -f * wbi}};
+  }
+  LinkIO<double>::st(a.gstep, gi, gg);
+  if (a.omega_out) {
+    double* o = a.omega_out + gi * 3;
+    o[0] = (double)w3;
+    o[1] = (double)wbr;
+    o[2] = (double)wbi;
+  }
+}
+
 template <typename R, int LOGN, bool CG = false>
 __global__ void __launch_bounds__(kFaThreads) fa_g_kernel(FaArgs a) {
   using G = FaLines<LOGN>;
-  constexpr int n = G::n, ld = G::ld, NL = G::NLT / 2;
+  constexpr int n = G::n, NL = G::NLT / 2, ld = kFaDirect<LOGN> ? G::ldx : G::ld;
   extern __shared__ __align__(16) FftC fa_sm[];
   FftC* d = fa_sm;
   FftC* tw = d + G::NLT * ld;
@@ -485,44 +678,81 @@ __global__ void __launch_bounds__(kFaThreads) fa_g_kernel(FaArgs a) {
   const FftC* F = reinterpret_cast<const FftC*>(a.fft);
   const int lg0 = a.zg0 * a.L[1];
   load_twiddles(tw, a.tw, n, +1);
-  for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
-    const int j = e >> LOGN, k = e & (n - 1), l = l0 + j;
-    const size_t gi = l < nlines ? nat_index<0>(a, lg0 + l, k) : 0;
-    d[j * ld + k] = l < nlines ? F[gi] : FftC{0, 0};
-    d[(NL + j) * ld + k] = l < nlines ? F[V + gi] : FftC{0, 0};
+  if constexpr (kFaDirect<LOGN>) {
+    // step 1 from global memory, columns to consecutive threads (runs of N2
+    // points)
+    constexpr int N1 = G::N1, N2 = G::N2, NLT = G::NLT;
+    static_assert(NLT * N2 <= kFaThreads, "one column per thread");
+    FftC r[N1];
+    const int n2 = threadIdx.x % N2, j1 = threadIdx.x / N2, l1 = l0 + (j1 & (NL - 1));
+    if (j1 < NLT) {
+      const FftC* Fl = F + (j1 >= NL ? V : 0) + nat_index<0>(a, lg0 + (l1 < nlines ? l1 : 0), n2);
+#pragma unroll
+      for (int i = 0; i < N1; ++i) r[i] = l1 < nlines ? Fl[i * N2] : FftC{0, 0};
+    }
+    __syncthreads();  // the twiddles
+    if (j1 < NLT) {
+      fft_step1<LOGN>(r, n2, tw);
+      fft_put_column<LOGN>(d + j1 * ld, n2, r);
+    }
+    __syncthreads();
+    constexpr int IB = NLT * N1 / kFaThreads;
+    FftC w[IB][N2];
+#pragma unroll
+    for (int q = 0; q < IB; ++q) {
+      const int it = threadIdx.x + q * kFaThreads;
+      fft_step2<LOGN>(d + (it / N1) * ld, it % N1, w[q], tw);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < IB; ++q) {
+      const int it = threadIdx.x + q * kFaThreads;
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) d[(it / N1) * ld + it % N1 + N1 * k2] = w[q][k2];
+    }
+  } else {
+    for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
+      const int j = e >> LOGN, k = e & (n - 1), l = l0 + j;
+      const size_t gi = l < nlines ? nat_index<0>(a, lg0 + l, k) : 0;
+      d[j * ld + k] = l < nlines ? F[gi] : FftC{0, 0};
+      d[(NL + j) * ld + k] = l < nlines ? F[V + gi] : FftC{0, 0};
+    }
+    __syncthreads();
+    fft2_lines<LOGN>(d, tw);
   }
   __syncthreads();
-  fft2_lines<LOGN>(d, tw);
-  for (int e = threadIdx.x; e < NL * n; e += blockDim.x) {
-    const int j = e >> LOGN, x = e & (n - 1), l = l0 + j;
-    if (l >= nlines) continue;
-    const int y = l & (a.L[1] - 1), z = (l >> a.logL[1]) + a.zl0;
-    const int p = (x + y + z) & 1, s = site_index(x, y, z, ch.hx, ch.nxy);
-    const double w3 = d[(NL + j) * ld + x].x, wbr = d[j * ld + x].x, wbi = d[j * ld + x].y;
-    if (CG) {
-      const double beta = a.cg->beta;
-      const size_t V2 = 2 * (size_t)ch.nh, gi = (size_t)p * ch.nh + s;
-      float* S = a.sdir;
+  // the sites, four at a time per thread: the old direction's loads of a batch
+  // are in flight together (its stores may not be passed by later loads).  128^3
+  // 39.7 -> 18.6 us, 256^3 134 us (5.0 TB/s).
+  constexpr int kBatch = 4;
+  const double beta = CG ? a.cg->beta : 0.0;
+  const size_t V2 = 2 * (size_t)ch.nh;
+  for (int e0 = threadIdx.x; e0 < NL * n; e0 += kBatch * kFaThreads) {
+    size_t gi[kBatch];
+    float so[kBatch][3];
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q) {
+      const int e = e0 + q * kFaThreads, j = e >> LOGN, x = e & (n - 1), l = l0 + j;
+      const int y = l & (a.L[1] - 1), z = (l >> a.logL[1]) + a.zl0;
+      gi[q] = (size_t)((x + y + z) & 1) * ch.nh + site_index(x, y, z, ch.hx, ch.nxy);
       // beta = 0 starts afresh (the old direction is not read)
-      S[gi] = (float)(beta > 0.0 ? w3 + beta * (double)S[gi] : w3);
-      S[V2 + gi] = (float)(beta > 0.0 ? wbr + beta * (double)S[V2 + gi] : wbr);
-      S[2 * V2 + gi] = (float)(beta > 0.0 ? wbi + beta * (double)S[2 * V2 + gi] : wbi);
-      continue;
+      if (CG && beta > 0.0 && e < NL * n && l < nlines) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) so[q][c] = __ldcg(a.sdir + c * V2 + gi[q]);
+      }
     }
-    const double nw = sqrt(w3 * w3 + wbr * wbr + wbi * wbi);
-    su2<double> gg{{1.0, 0.0}, {0.0, 0.0}};
-    if (nw > 0.0) {
-      double sn, cs;
-      sincos(nw, &sn, &cs);
-      const double f = sn / nw;
-      gg = su2<double>{{cs, -f * w3}, {-f * wbr, -f * wbi}};
-    }
-    LinkIO<double>::st(a.gstep, (size_t)p * ch.nh + s, gg);
-    if (a.omega_out) {
-      double* o = a.omega_out + ((size_t)p * ch.nh + s) * 3;
-      o[0] = (double)w3;
-      o[1] = (double)wbr;
-      o[2] = (double)wbi;
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q) {
+      const int e = e0 + q * kFaThreads, j = e >> LOGN, x = e & (n - 1);
+      if (e >= NL * n || l0 + j >= nlines) continue;
+      const double w3 = d[(NL + j) * ld + x].x, wbr = d[j * ld + x].x, wbi = d[j * ld + x].y;
+      if (CG) {
+        a.sdir[gi[q]] = (float)(beta > 0.0 ? w3 + beta * (double)so[q][0] : w3);
+        a.sdir[V2 + gi[q]] = (float)(beta > 0.0 ? wbr + beta * (double)so[q][1] : wbr);
+        a.sdir[2 * V2 + gi[q]] = (float)(beta > 0.0 ? wbi + beta * (double)so[q][2] : wbi);
+      } else {
+        fa_site_g(a, gi[q], w3, wbr, wbi);
+      }
     }
   }
 }
@@ -547,9 +777,7 @@ __device__ __forceinline__ su2<double> fa_exp_dir(const float* S, size_t V2, siz
   return su2<double>{{c, -f * w3}, {-f * wbr, -f * wbi}};
 }
 
-// CG: g(x) = exp(alpha X(x)) per site.  (Forming it inside the apply kernel
-// instead, four exponentials per site, took 108 us against 17 + 69 us at
-// 128^3 for the first iterations from G = 1, whose large angles take sincos.)
+// CG on z-slabs: g(x) = exp(alpha X(x)) per site
 __global__ void __launch_bounds__(kBlock) fa_gstep_kernel(FaArgs a) {
   if (fa_done(a)) return;
   const int i = blockIdx.x * kBlock + threadIdx.x;
@@ -557,26 +785,17 @@ __global__ void __launch_bounds__(kBlock) fa_gstep_kernel(FaArgs a) {
   LinkIO<double>::st(a.gstep, (size_t)i, fa_exp_dir(a.sdir, 2 * (size_t)a.ch->nh, (size_t)i, a.cg->alpha));
 }
 
-// (7) U_f(x,mu) -> g(x) U_f(x,mu) g(x+mu)^+, A_f -> g A_f g^+, G -> g G
-template <typename R>
-__global__ void __launch_bounds__(kBlock) fa_apply_kernel(FaArgs a) {
-  if (fa_done(a)) return;
-  const ChainDev& ch = *a.ch;
-  const int i = blockIdx.x * kBlock + threadIdx.x;
-  const int nvis = ch.nh - 2 * a.s_lo;  // visited sites per parity
-  if (i >= 2 * nvis) return;
-  const int eo = i >= nvis ? 1 : 0, oe = 1 - eo, s = a.s_lo + i - eo * nvis, nh = ch.nh;
-  const Coord X = site_coord(eo, s, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
-  const su2<double> gx = LinkIO<double>::ld_cg(a.gstep, (size_t)eo * nh + s);
-  const int L[3] = {ch.L1, ch.L2, ch.L3};
+// U_f(x,mu) -> g(x) U_f(x,mu) g(x+mu)^+, A_f -> g A_f g^+, G -> g G at one site,
+// gp(mu) = g(x+mu) (straight-line code: a branch inside changes how the FP64
+// products are contracted, and with it the last bits)
+template <typename R, typename GP>
+__device__ __forceinline__ void fa_apply_site(const FaArgs& a, const ChainDev& ch, int eo, int s, su2<double> gx,
+                                              GP gp) {
+  const int nh = ch.nh;
 #pragma unroll
   for (int mu = 0; mu < 3; ++mu) {
-    int c[3] = {X.x, X.y, X.z};
-    c[mu] = wrap(c[mu] + 1, L[mu]);
-    const int sp = site_index(c[0], c[1], c[2], ch.hx, ch.nxy);
-    const su2<double> gp = LinkIO<double>::ld_cg(a.gstep, (size_t)oe * nh + sp);
     const size_t li = ((size_t)(mu * 2 + eo)) * nh + s;
-    LinkIO<R>::st(ch.uf, li, to_r<R>(unitarise64(nd(nn(gx, to_d(LinkIO<R>::ld_cg(ch.uf, li))), gp))));
+    LinkIO<R>::st(ch.uf, li, to_r<R>(unitarise64(nd(nn(gx, to_d(LinkIO<R>::ld_cg(ch.uf, li))), gp(mu)))));
   }
   R* Af = reinterpret_cast<R*>(ch.af);
   const su2<double> t =
@@ -590,18 +809,98 @@ __global__ void __launch_bounds__(kBlock) fa_apply_kernel(FaArgs a) {
     LinkIO<R>::st(ch.g, gi, to_r<R>(unitarise64(nn(gx, to_d(LinkIO<R>::ld_cg(ch.g, gi))))));
   }
 }
+// a site's fields into L2 ahead of fa_apply_site
+template <typename R>
+__device__ __forceinline__ void fa_prefetch_site(const FaArgs& a, const ChainDev& ch, int eo, int s) {
+  auto pf = [](const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
+#pragma unroll
+  for (int mu = 0; mu < 3; ++mu)
+    pf(static_cast<const char*>(ch.uf) + (((size_t)(mu * 2 + eo)) * ch.nh + s) * LinkIO<R>::kBytes);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) pf(reinterpret_cast<const R*>(ch.af) + ((size_t)(eo * 3 + k)) * ch.nh + s);
+  if (a.track) pf(static_cast<const char*>(ch.g) + ((size_t)eo * ch.nh + s) * LinkIO<R>::kBytes);
+}
+
+// (7) g (in memory) applied at the visited sites
+template <typename R>
+__global__ void __launch_bounds__(kBlock) fa_apply_kernel(FaArgs a) {
+  if (fa_done(a)) return;
+  const ChainDev& ch = *a.ch;
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  const int nvis = ch.nh - 2 * a.s_lo;  // visited sites per parity
+  if (i >= 2 * nvis) return;
+  const int eo = i >= nvis ? 1 : 0, oe = 1 - eo, s = a.s_lo + i - eo * nvis;
+  const Coord X = site_coord(eo, s, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
+  const NbrOff o = nbr_offsets(ch, X);
+  fa_apply_site<R>(a, ch, eo, s, LinkIO<double>::ld_cg(a.gstep, (size_t)eo * ch.nh + s), [&](int mu) {
+    return LinkIO<double>::ld_cg(a.gstep, (size_t)oe * ch.nh + (s + o.p[mu]));
+  });
+}
+
+// CG on an undecomposed lattice: g = exp(alpha X) formed and applied in one
+// kernel.  A block takes a tile of at most 16 x 4 x 4 sites (2^l0 x 2^l1 x
+// 2^l2), one per thread: it prefetches the sites' fields, forms g at the sites
+// and at those above them along each axis (1.56 exponentials per site) in
+// shared memory while they arrive in L2, and applies it.  g in memory between two kernels
+// (FP64: 32 bytes per site, written once and read at four sites) took 19 + 87
+// us at 128^3, this 88; four sites per thread of a 64 x 4 x 4 tile, loading
+// each after the last, 101; the four exponentials of a site in its own thread
+// 108.
+constexpr int kFaTileLog[3] = {4, 2, 2};
+template <typename R>
+__global__ void __launch_bounds__(kBlock) fa_exp_apply_kernel(FaArgs a, int l0, int l1, int l2) {
+  extern __shared__ __align__(16) double fa_gs[];  // four planes of np components
+  if (fa_done(a)) return;
+  const ChainDev& ch = *a.ch;
+  const int S = 1 << l0, T = 1 << l1, U = 1 << l2, nm = S * T * U;
+  const int hx0 = nm, hy0 = hx0 + T * U, hz0 = hy0 + S * U, np = hz0 + S * T;
+  const int b = blockIdx.x, bx = b & ((a.L[0] >> l0) - 1), by = (b >> (a.logL[0] - l0)) & ((a.L[1] >> l1) - 1),
+            bz = b >> (a.logL[0] - l0 + a.logL[1] - l1);
+  const int x0 = bx << l0, y0 = by << l1, z0 = bz << l2;
+  const int i = threadIdx.x, xx = i & (S - 1), yy = (i >> l0) & (T - 1), zz = i >> (l0 + l1);
+  const int eo = (x0 + xx + y0 + yy + z0 + zz) & 1, s = site_index(x0 + xx, y0 + yy, z0 + zz, ch.hx, ch.nxy);
+  if (i < nm) fa_prefetch_site<R>(a, ch, eo, s);
+  const size_t V2 = 2 * (size_t)ch.nh;
+  const double al = a.cg->alpha;
+  for (int p = i; p < np; p += kBlock) {
+    // point p: the sites, then their neighbours past the tile along x, y, z
+    int x = xx, y = yy, z = zz;
+    if (p >= hz0) x = (p - hz0) & (S - 1), y = (p - hz0) >> l0, z = U;
+    else if (p >= hy0) x = (p - hy0) & (S - 1), y = T, z = (p - hy0) >> l0;
+    else if (p >= hx0) x = S, y = (p - hx0) & (T - 1), z = (p - hx0) >> l1;
+    x = (x0 + x) & (a.L[0] - 1), y = (y0 + y) & (a.L[1] - 1), z = (z0 + z) & (a.L[2] - 1);
+    const size_t gi = (size_t)((x + y + z) & 1) * ch.nh + site_index(x, y, z, ch.hx, ch.nxy);
+    const su2<double> g = fa_exp_dir(a.sdir, V2, gi, al);
+    fa_gs[p] = g.a.re;
+    fa_gs[np + p] = g.a.im;
+    fa_gs[2 * np + p] = g.b.re;
+    fa_gs[3 * np + p] = g.b.im;
+  }
+  __syncthreads();
+  if (i >= nm) return;
+  auto g_at = [&](int p) {
+    return su2<double>{{fa_gs[p], fa_gs[np + p]}, {fa_gs[2 * np + p], fa_gs[3 * np + p]}};
+  };
+  const int up[3] = {xx + 1 < S ? i + 1 : hx0 + zz * T + yy, yy + 1 < T ? i + S : hy0 + zz * S + xx,
+                     zz + 1 < U ? i + S * T : hz0 + yy * S + xx};
+  fa_apply_site<R>(a, ch, eo, s, g_at(i), [&](int mu) { return g_at(up[mu]); });
+}
+template <typename R>
+void launch_fa_exp_apply(const FaArgs& a, cudaStream_t s) {
+  int lt[3];
+  static_assert(kFaTileLog[0] + kFaTileLog[1] + kFaTileLog[2] == 8 && kBlock == 256, "one site per thread");
+  for (int d = 0; d < 3; ++d) lt[d] = std::min(kFaTileLog[d], a.logL[d]);
+  const int S = 1 << lt[0], T = 1 << lt[1], U = 1 << lt[2];
+  const size_t smem = (size_t)(S * T * U + T * U + S * U + S * T) * 4 * sizeof(double);
+  const int nb = 1 << (a.logL[0] + a.logL[1] + a.logL[2] - lt[0] - lt[1] - lt[2]);
+  fa_exp_apply_kernel<R><<<nb, kBlock, smem, s>>>(a, lt[0], lt[1], lt[2]);
+}
 
 // CG: beta = max(0, (S_k - C_k) / S_(k-1)) from the scale kernel's sums
 __global__ void __launch_bounds__(1024) fa_beta_kernel(FaArgs a, int nparts) {
   if (fa_done(a)) return;
-  double v[2] = {0.0, 0.0};
-  for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
-    v[0] += a.cgpart[2 * b];
-    v[1] += a.cgpart[2 * b + 1];
-  }
   __shared__ double t[2];
-  block_reduce_store<2>(v, t);
-  __syncthreads();
+  fa_sums<2>(a.cgpart, nparts, t);
   if (threadIdx.x == 0) {
     FaCg* g = a.cg;
     double beta = 0.0;
@@ -665,15 +964,8 @@ __global__ void __launch_bounds__(kBlock) fa_line_kernel(FaArgs a) {
 // that does not ascend moves nothing; both restart from the gradient.
 __global__ void __launch_bounds__(1024) fa_alpha_kernel(FaArgs a, int nparts) {
   if (fa_done(a)) return;
-  double v[3] = {0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
-    v[0] += a.cgpart[3 * b];
-    v[1] += a.cgpart[3 * b + 1];
-    v[2] += a.cgpart[3 * b + 2];
-  }
   __shared__ double t[3];
-  block_reduce_store<3>(v, t);
-  __syncthreads();
+  fa_sums<3>(a.cgpart, nparts, t);
   if (threadIdx.x == 0) {
     FaCg* g = a.cg;
     const double nh = a.nh_all > 0.0 ? a.nh_all : (double)a.ch->nh;
@@ -795,7 +1087,9 @@ void fa_div_launch(const FaArgs& a, int nb, cudaStream_t s) {
 }
 template <typename R, int LOGN, bool CG = false>
 void fa_g_launch(const FaArgs& a, int nb, cudaStream_t s) {
-  fa_launch(fa_g_kernel<R, LOGN, CG>, "fa_g_kernel", LOGN, dim3(nb), FaLines<LOGN>::smem(1, 0), a, s);
+  using G = FaLines<LOGN>;
+  fa_launch(fa_g_kernel<R, LOGN, CG>, "fa_g_kernel", LOGN, dim3(nb), G::smem(1, 0, kFaDirect<LOGN> ? G::ldx : G::ld), a,
+            s);
 }
 template <int AX, int SIGN, bool SCALE, int LOGN, bool CG = false>
 void fa_fft_launch(const FaArgs& a, int nb, cudaStream_t s) {
@@ -825,7 +1119,7 @@ int fa_blocks(long nlines, int logn, int fields) {
 }
 
 // enqueue one Fourier-accelerated iteration (kernels 1-7; cg: the
-// conjugate-gradient form, 11 kernels)
+// conjugate-gradient form, 10 kernels)
 template <typename R>
 void launch_fa_iteration(const ChainDev* chd, const ChainDev& ch, ChainState* cst, double gamma, void* buf,
                          size_t vcap, double* part, double* omega_out, int track, bool with_check, bool with_apply,
@@ -883,7 +1177,8 @@ void launch_fa_iteration(const ChainDev* chd, const ChainDev& ch, ChainState* cs
 #undef LCE_FA_GC
     fa_line_kernel<R><<<nbv, kBlock, 0, s>>>(a);
     fa_alpha_kernel<<<1, 1024, 0, s>>>(a, nbv);
-    fa_gstep_kernel<<<nbv, kBlock, 0, s>>>(a);
+    if (with_apply) launch_fa_exp_apply<R>(a, s);
+    return;
   } else {
 #define LCE_FA_G(L) fa_g_launch<R, L>(a, nbd, s)
     LCE_FA_SWITCH(a.logL[0], LCE_FA_G)

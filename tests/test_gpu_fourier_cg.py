@@ -101,3 +101,37 @@ def test_cg_in_a_batch_of_uneven_volumes():
             th, itf, itp = ens.landau_gauge_fourier(start, chain=c)
             assert th <= 1e-10
         ens.sweeps(2, 0)
+
+
+# lines of 32 to 512 points take the transforms that read and write global
+# memory in their steps, shorter and longer ones the other form, on each axis;
+# extents below and above the 16 x 4 x 4 tile of the kernel that forms and
+# applies g; lattices of less than one block of lines
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("L", [(2, 2, 2), (32, 2, 4), (2, 64, 16), (4, 2, 128), (256, 8, 2), (8, 256, 4), (2, 4, 512),
+                               (512, 2, 2), (2, 512, 2), (16, 1024, 2), (1024, 4, 2), (4, 4, 1024), (64, 32, 16)])
+def test_cg_steps_at_tile_and_line_edges(precision, L):
+    """Directions against NumPy's FFT (the tolerance of test_gpu_fourier.py: FP32
+    transforms times the longest wavelength's 1/p^2), and a few CG steps: the
+    functional rises and U_f, A_f are the tracked G applied to U, A (each step
+    rounds links, A and G to the fields' precision: 6 steps, a few ulps each)."""
+    from lceqcd_b200 import Lattice, LceError
+    from test_gpu_fourier import numpy_direction
+    g = Lattice(L, **COUP, limit_or=1e-30, seed=3, precision=precision, alpha=0.875)
+    g.init_hot(11)
+    g.sweeps(10, 0)
+    u, a = g.download()
+    g.upload(u, a, which=1)
+    om = g.debug_fourier_step(1.0)
+    ref, _ = numpy_direction(np.asarray(u, np.float64), L, 0.875, 1.0)
+    assert np.abs(om - ref).max() <= max(5e-6, 1e-10 * max(L) ** 2) * max(1.0, np.abs(ref).max())
+    F0 = g.gauge_functional()
+    with pytest.raises(LceError):
+        g.landau_gauge_fourier_cg("identity", max_iters=6)
+    assert g.gauge_functional() > F0
+    uf, af = g.download(which=1)
+    g.apply_transform()
+    ur, ar = g.download(which=1)
+    tol = 40 * np.finfo(uf.dtype).eps
+    assert np.abs(uf - ur).max() <= tol and np.abs(af - ar).max() <= tol * max(1.0, np.abs(af).max())
+    g.close()
