@@ -410,7 +410,6 @@ int enq_pass(lce_ctx* c, Enq& q, size_t i) {
   // earlier queue's finalize may still be advancing the RNG counters); the
   // later passes follow pass kernels of this queue only
   a.rng_early = i > 0 ? 1 : 0;
-  a.trigger_late = i == 0 ? 1 : 0;
   // level 1 of the previous pass's slot in extra blocks of this launch
   a.ntiles = nblocks;
   int grid = nblocks;
@@ -506,7 +505,6 @@ int enqueue_persistent(lce_ctx* c, const std::vector<unsigned char>& routines, i
   b.site_off = c->site_off;
   b.stream_nh = c->stream_nh;
   b.rng_early = 0;
-  b.trigger_late = 0;
   FinalizeArgs& f = a.fin;
   f.chains = c->ch_d;
   f.blk_begin = c->blk_d;
@@ -973,6 +971,8 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
       return bail(e, "cudaMemcpy(state)");
   }
   c->scratch_n = (size_t)2 * ceil_div(2L * c->max_nh, 256) + (size_t)32 * c->max_L3 + 64;
+  // gauge fixing: at most 1024 theta partials of small blocks
+  c->scratch_n = std::max(c->scratch_n, (size_t)1024);
   // slice measurements: sums, output and the segments' partial sums
   for (const ChainDev& d : c->ch)
     c->scratch_n = std::max(c->scratch_n, (size_t)21 * d.L3 + 5 + slice_part_doubles(d.nxy, d.L3));
@@ -1028,18 +1028,10 @@ int gf_loop(lce_ctx* c, int chain, double* theta, int* iters, int max_iters, int
     if (it == c->gf_exec.end()) {
       cudaGraph_t g;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < batch; ++k) {
-        if (it_flags >= 0) {
-          if (c->prec == LCE_PREC_F64)
-            launch_it_iteration<double>(c->ch_d + chain, c->cst_d + chain, it_flags, 1, part, ch.nh, c->stream);
-          else
-            launch_it_iteration<float>(c->ch_d + chain, c->cst_d + chain, it_flags, 1, part, ch.nh, c->stream);
-        } else if (c->prec == LCE_PREC_F64) {
-          launch_gf_iteration<double>(c->ch_d + chain, c->cst_d + chain, track, part, ch.nh, c->stream);
-        } else {
-          launch_gf_iteration<float>(c->ch_d + chain, c->cst_d + chain, track, part, ch.nh, c->stream);
-        }
-      }
+      if (c->prec == LCE_PREC_F64)
+        launch_gf_batch<double>(c->ch_d + chain, c->cst_d + chain, track, it_flags, part, ch.nh, batch, c->stream);
+      else
+        launch_gf_batch<float>(c->ch_d + chain, c->cst_d + chain, track, it_flags, part, ch.nh, batch, c->stream);
       CK(cudaStreamEndCapture(c->stream, &g));
       cudaGraphExec_t ex;
       cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
@@ -2308,9 +2300,9 @@ int lce_it_gauge_fixing(lce_ctx* c, int chain, double step, int flags, double* d
   CK(cudaMemcpyAsync(c->cst_d + chain, &cs, sizeof(cs), cudaMemcpyHostToDevice, c->stream));
   // the subroutine itself: no reunitarisation
   if (c->prec == LCE_PREC_F64)
-    launch_it_iteration<double>(c->ch_d + chain, c->cst_d + chain, flags, 0, c->scratch_d, ch.nh, c->stream);
+    launch_it_iteration<double>(c->ch_d + chain, c->cst_d + chain, flags, c->scratch_d, ch.nh, c->stream);
   else
-    launch_it_iteration<float>(c->ch_d + chain, c->cst_d + chain, flags, 0, c->scratch_d, ch.nh, c->stream);
+    launch_it_iteration<float>(c->ch_d + chain, c->cst_d + chain, flags, c->scratch_d, ch.nh, c->stream);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(&cs, c->cst_d + chain, sizeof(cs), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

@@ -27,6 +27,12 @@ __device__ __forceinline__ su2<R> ldUf(const ChainDev& ch, int mu, int p, int s)
   return LinkIO<R>::ld_cg(ch.uf, ((size_t)(mu * 2 + p)) * ch.nh + s);
 }
 
+// A value the compiler takes as new here.  The FP32 products of a value that
+// was loaded in an earlier block are contracted otherwise than those of one
+// loaded beside them; A_f, loaded early, keeps the bits it always had.
+__device__ __forceinline__ void opaque(float& x) { asm volatile("" : "+f"(x)); }
+__device__ __forceinline__ void opaque(double& x) { asm volatile("" : "+d"(x)); }
+
 template <int MU>
 __device__ __forceinline__ int nbr_dn(const ChainDev& ch, Coord X) {
   int x = X.x, y = X.y, z = X.z;
@@ -60,6 +66,34 @@ __device__ __forceinline__ void gf_sums(const ChainDev& ch, const su2<R> (&um)[3
   t2.b = t2.b + mk<double>(al * ud[2].b.re, al * ud[2].b.im);
 }
 
+// The check of the previous iteration, made by every block of an iteration's
+// first half-step for itself (nprev partials; 0: a check kernel follows every
+// iteration), so that a batch needs no one-block kernel between iterations:
+// the blocks add the partials in the same order and agree.  Block 0 records a
+// stop.  gf_iters is counted by the second half-step, so it stands still here;
+// 0: nothing to check yet.  A batch ends with gf_check_kernel, which gives the
+// host the state of its last iteration.
+__device__ __forceinline__ bool gf_stops(const ChainDev& ch, const ChainState* cst, double theta, int it) {
+  return !(theta > ch.limit_or) || (cst->gf_cap > 0 && it >= cst->gf_cap);
+}
+template <int BS>
+__device__ __forceinline__ bool gf_prev_stops(const ChainDev& ch, ChainState* cst, const double* part, int nprev) {
+  const int it = cst->gf_iters;
+  __shared__ double tot;
+  double v[1] = {0.0};
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nprev; b += BS) v[0] += __ldcg(part + b);
+  block_reduce_store<1>(v, &tot);
+  __syncthreads();
+  const double theta = tot / ch.nh;
+  if (it == 0 || !gf_stops(ch, cst, theta, it)) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    cst->gf_theta = theta;
+    cst->gf_done = 1;
+  }
+  return true;
+}
+
 // track != 0: also accumulate the gauge transform, G(x) -> Omega(x) G(x), so
 // that U_f(x,mu) = G(x) U(x,mu) G(x+mu)^+ holds throughout.  FP32 is held to
 // 64 registers (4 blocks per SM; 68 allowed 3): 8.5% less time per
@@ -68,25 +102,43 @@ __device__ __forceinline__ void gf_sums(const ChainDev& ch, const su2<R> (&um)[3
 // [s_lo, nh - s_lo) are visited), 0 for a whole lattice.  last: the
 // iteration's second half-step (the whole lattice's odd sites; a slab's
 // local parity eo may be flipped), which sums theta and reunitarises.
-template <typename R>
-__global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 1)
-    gf_half_kernel(const ChainDev* chp, const ChainState* cst, int eo, double* part, int track, int s_lo, int last) {
-  pdl_trigger();
+// BS: threads per block (gf_block).  nprev: gf_prev_stops (first half-step).
+template <typename R, int BS>
+__global__ void __launch_bounds__(BS, sizeof(R) == 4 ? 4 * kBlock / BS : 1)
+    gf_half_kernel(const ChainDev* chp, ChainState* cst, int eo, double* part, int track, int s_lo, int last,
+                   int nprev) {
   const ChainDev& ch = *chp;
-  const int s = s_lo + blockIdx.x * kBlock + threadIdx.x;
+  const int s = s_lo + blockIdx.x * BS + threadIdx.x;
   const int oe = 1 - eo, nh = ch.nh, s_hi = nh - s_lo;
   const Coord X = site_coord(eo, s < s_hi ? s : s_lo, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
   const int xm[3] = {nbr_dn<0>(ch, X), nbr_dn<1>(ch, X), nbr_dn<2>(ch, X)};
   pdl_wait();
-  if (cst->gf_done) return;
+  // every load of the half-step before the first branch on one: a chain of
+  // round trips to L2 is what a small lattice's half-step waits for
   double th[1] = {0.0};
+  su2<R> um[3], ud[3];
+  R a1 = (R)0, a2 = (R)0, a3 = (R)0;
+  R* Af = reinterpret_cast<R*>(ch.af);
   if (s < s_hi) {
-    su2<R> um[3], ud[3];
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
       um[mu] = ldUf<R>(ch, mu, eo, s);
       ud[mu] = ldUf<R>(ch, mu, oe, xm[mu]);
     }
+    a1 = __ldcg(Af + ((size_t)(eo * 3 + 0)) * nh + s);
+    a2 = __ldcg(Af + ((size_t)(eo * 3 + 1)) * nh + s);
+    a3 = __ldcg(Af + ((size_t)(eo * 3 + 2)) * nh + s);
+  }
+  const int done = cst->gf_done;
+  const bool stop = !last && nprev && gf_prev_stops<BS>(ch, cst, part, nprev);
+  // Dependents may launch from here on.  Triggered at the kernel's start, the
+  // blocks of many waiting half-steps filled the SMs and a half-step's own
+  // blocks landed together on the few slots the last one left: 48 x 40 x 36
+  // 12.0 us per iteration against 7.5.
+  pdl_trigger();
+  if (done || stop) return;
+  if (last && nprev && blockIdx.x == 0 && threadIdx.x == 0) cst->gf_iters += 1;
+  if (s < s_hi) {
     su2<double> t1, t2;
     gf_sums<R>(ch, um, ud, t1, t2);
     // (:145-146) w = first row of sum [U + U^+(x-mu)]
@@ -128,9 +180,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 1)
       }
     }
     // (:243-252) A_f(x) -> Omega (iA) Omega^+
-    R* Af = reinterpret_cast<R*>(ch.af);
-    const R a1 = Af[((size_t)(eo * 3 + 0)) * nh + s], a2 = Af[((size_t)(eo * 3 + 1)) * nh + s],
-            a3 = Af[((size_t)(eo * 3 + 2)) * nh + s];
+    opaque(a1);
+    opaque(a2);
+    opaque(a3);
     const su2<R> ta = nn(o, ad(a1, a2, a3, o));
     Af[((size_t)(eo * 3 + 0)) * nh + s] = ta.b.im;
     Af[((size_t)(eo * 3 + 1)) * nh + s] = ta.b.re;
@@ -166,26 +218,42 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 1)
 // iteration, as f/landau_gauge.f:56-57 does for the overrelaxed form).
 // s_lo and last as for gf_half_kernel (a z-slab's visited sites; the whole
 // lattice's second half-step, which sums |g|^2 and reunitarises).
-template <typename R>
-__global__ void __launch_bounds__(kBlock) it_half_kernel(const ChainDev* chp, const ChainState* cst, int eo,
-                                                         double* part, int flags, int renorm, int s_lo, int last) {
-  pdl_trigger();
+template <typename R, int BS>
+__global__ void __launch_bounds__(BS) it_half_kernel(const ChainDev* chp, ChainState* cst, int eo, double* part,
+                                                     int flags, int renorm, int s_lo, int last, int nprev) {
   const ChainDev& ch = *chp;
-  const int s = s_lo + blockIdx.x * kBlock + threadIdx.x;
+  const int s = s_lo + blockIdx.x * BS + threadIdx.x;
   const int oe = 1 - eo, nh = ch.nh, s_hi = nh - s_lo;
   const Coord X = site_coord(eo, s < s_hi ? s : s_lo, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
   const int xm[3] = {nbr_dn<0>(ch, X), nbr_dn<1>(ch, X), nbr_dn<2>(ch, X)};
   pdl_wait();
-  if (cst->gf_done) return;
+  // every load of the half-step before the first branch on one: a chain of
+  // round trips to L2 is what a small lattice's half-step waits for
   double th[1] = {0.0};
+  su2<R> um[3], ud[3];
+  R a1 = (R)0, a2 = (R)0, a3 = (R)0;
+  R* Af = reinterpret_cast<R*>(ch.af);
   if (s < s_hi) {
-    su2<R> um[3], ud[3];
-    double g1a = 0, g1br = 0, g1bi = 0, g2a = 0, g2br = 0, g2bi = 0;
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
       um[mu] = ldUf<R>(ch, mu, eo, s);
       ud[mu] = ldUf<R>(ch, mu, oe, xm[mu]);
     }
+    a1 = __ldcg(Af + ((size_t)(eo * 3 + 0)) * nh + s);
+    a2 = __ldcg(Af + ((size_t)(eo * 3 + 1)) * nh + s);
+    a3 = __ldcg(Af + ((size_t)(eo * 3 + 2)) * nh + s);
+  }
+  const int done = cst->gf_done;
+  const bool stop = !last && nprev && gf_prev_stops<BS>(ch, cst, part, nprev);
+  // Dependents may launch from here on.  Triggered at the kernel's start, the
+  // blocks of many waiting half-steps filled the SMs and a half-step's own
+  // blocks landed together on the few slots the last one left: 48 x 40 x 36
+  // 12.0 us per iteration against 7.5.
+  pdl_trigger();
+  if (done || stop) return;
+  if (last && nprev && blockIdx.x == 0 && threadIdx.x == 0) cst->gf_iters += 1;
+  if (s < s_hi) {
+    double g1a = 0, g1br = 0, g1bi = 0, g2a = 0, g2br = 0, g2bi = 0;
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
       g1a += (double)um[mu].a.im;
@@ -209,9 +277,9 @@ __global__ void __launch_bounds__(kBlock) it_half_kernel(const ChainDev* chp, co
     // the reference divides 0 by 0 where g = 0; the limit is 1
     const double t2 = t1 > 0.0 ? sin(t1) / t1 : 1.0;
     const su2<R> o{{(R)cos(t1), (R)(ha * t2)}, {(R)(hbr * t2), (R)(hbi * t2)}};
-    R* Af = reinterpret_cast<R*>(ch.af);
-    const R a1 = Af[((size_t)(eo * 3 + 0)) * nh + s], a2 = Af[((size_t)(eo * 3 + 1)) * nh + s],
-            a3 = Af[((size_t)(eo * 3 + 2)) * nh + s];
+    opaque(a1);
+    opaque(a2);
+    opaque(a3);
     const su2<R> ta = nn(o, ad(a1, a2, a3, o));
     Af[((size_t)(eo * 3 + 0)) * nh + s] = ta.b.im;
     Af[((size_t)(eo * 3 + 1)) * nh + s] = ta.b.re;
@@ -270,9 +338,10 @@ __global__ void transform_identity_kernel(void* g, size_t n) {
     LinkIO<R>::st(g, i, su2<R>{{(R)1, (R)0}, {(R)0, (R)0}});
 }
 
-// sum the theta partials in block order, count the iteration, test convergence
+// sum the theta partials in block order, count the iteration (unless the
+// second half-step has), test convergence
 __global__ void __launch_bounds__(1024) gf_check_kernel(const ChainDev* chp, ChainState* cst, const double* part,
-                                                        int nblocks) {
+                                                        int nblocks, int count) {
   pdl_trigger();
   pdl_wait();
   if (cst->gf_done) return;
@@ -284,10 +353,10 @@ __global__ void __launch_bounds__(1024) gf_check_kernel(const ChainDev* chp, Cha
   __syncthreads();
   if (threadIdx.x == 0) {
     const double theta = tot / chp->nh;
-    const int it = cst->gf_iters + 1;
+    const int it = cst->gf_iters + count;
     cst->gf_iters = it;
     cst->gf_theta = theta;
-    if (!(theta > chp->limit_or) || (cst->gf_cap > 0 && it >= cst->gf_cap)) cst->gf_done = 1;
+    if (gf_stops(*chp, cst, theta, it)) cst->gf_done = 1;
   }
 }
 
@@ -351,20 +420,57 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* part, 
   block_reduce_store<NQ>(v, out);
 }
 
+// Threads per block of an undecomposed lattice's half-steps, and whether an
+// iteration's check is made by the next one's first half-step (gf_prev_stops).
+// 128 threads up to 8192 sites per parity, where blocks of 256 leave most of
+// the chip idle (16^3 6.97 -> 6.52 us per iteration, FP64 6.67 -> 5.45; at 48 x
+// 40 x 36 256 is better, 12.00 against 12.27).  Up to 1024 partials every block
+// can add them (64^3, 512 of them: an iteration 14.7 -> 12.9 us, 8^3 8.6 ->
+// 6.2); at 128^3, 4096, the check kernel's 4 of 82 us are the cheaper.
+constexpr int kGfSmallBlock = 128, kGfSmallSites = 8192, kGfMaxPartials = 1024;
+int gf_block(int nh) { return nh <= kGfSmallSites ? kGfSmallBlock : kBlock; }
+int gf_folds(int nh) {
+  const int nb = ceil_div(nh, gf_block(nh));
+  return nb <= kGfMaxPartials ? nb : 0;
+}
+
+// programmatic dependent launch: each kernel waits in griddepcontrol.wait
 template <typename R>
-void launch_gf_iteration(const ChainDev* ch, ChainState* cst, int track, double* part, int nh, cudaStream_t s) {
-  const int nb = ceil_div(nh, kBlock);
-  // programmatic dependent launch: each kernel waits in griddepcontrol.wait
-  (void)launch_pdl(gf_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, 0, part, track, 0, 0);
-  (void)launch_pdl(gf_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, 1, part, track, 0, 1);
-  (void)launch_pdl(gf_check_kernel, 1, 1024, 0, s, ch, cst, (const double*)part, nb);
+void gf_half(const ChainDev* ch, ChainState* cst, int eo, double* part, int track, int nh, cudaStream_t s) {
+  const int bs = gf_block(nh), nb = ceil_div(nh, bs);
+  auto* k = bs == kGfSmallBlock ? gf_half_kernel<R, kGfSmallBlock> : gf_half_kernel<R, kBlock>;
+  (void)launch_pdl(k, nb, bs, 0, s, ch, cst, eo, part, track, 0, eo, gf_folds(nh));
+}
+template <typename R>
+void it_half(const ChainDev* ch, ChainState* cst, int eo, double* part, int flags, int renorm, int nh, int nprev,
+             cudaStream_t s) {
+  const int bs = gf_block(nh), nb = ceil_div(nh, bs);
+  auto* k = bs == kGfSmallBlock ? it_half_kernel<R, kGfSmallBlock> : it_half_kernel<R, kBlock>;
+  (void)launch_pdl(k, nb, bs, 0, s, ch, cst, eo, part, flags, renorm, 0, eo, nprev);
+}
+void gf_check(const ChainDev* ch, ChainState* cst, const double* part, int nh, int count, cudaStream_t s) {
+  (void)launch_pdl(gf_check_kernel, 1, 1024, 0, s, ch, cst, part, ceil_div(nh, gf_block(nh)), count);
+}
+
+template <typename R>
+void launch_gf_batch(const ChainDev* ch, ChainState* cst, int track, int it_flags, double* part, int nh, int n,
+                     cudaStream_t s) {
+  const int folds = gf_folds(nh);
+  for (int k = 0; k < n; ++k) {
+    for (int eo = 0; eo < 2; ++eo) {
+      if (it_flags >= 0) it_half<R>(ch, cst, eo, part, it_flags, 1, nh, folds, s);
+      else gf_half<R>(ch, cst, eo, part, track, nh, s);
+    }
+    if (!folds) gf_check(ch, cst, part, nh, 1, s);
+  }
+  if (folds) gf_check(ch, cst, part, nh, 0, s);
 }
 
 template <typename R>
 int launch_gf_half(const ChainDev* ch, ChainState* cst, int eo, int last, double* part, int nh, int s_lo, int track,
                    cudaStream_t s) {
   const int nb = ceil_div(nh - 2 * s_lo, kBlock);
-  (void)launch_pdl(gf_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, eo, part, track, s_lo, last);
+  (void)launch_pdl(gf_half_kernel<R, kBlock>, nb, kBlock, 0, s, ch, cst, eo, part, track, s_lo, last, 0);
   return nb;
 }
 
@@ -374,12 +480,9 @@ void launch_gf_check_slabs(const ChainDev* ch, ChainState* cst, const double* su
 }
 
 template <typename R>
-void launch_it_iteration(const ChainDev* ch, ChainState* cst, int flags, int renorm, double* part, int nh,
-                         cudaStream_t s) {
-  const int nb = ceil_div(nh, kBlock);
-  (void)launch_pdl(it_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, 0, part, flags, renorm, 0, 0);
-  (void)launch_pdl(it_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, 1, part, flags, renorm, 0, 1);
-  (void)launch_pdl(gf_check_kernel, 1, 1024, 0, s, ch, cst, (const double*)part, nb);
+void launch_it_iteration(const ChainDev* ch, ChainState* cst, int flags, double* part, int nh, cudaStream_t s) {
+  for (int eo = 0; eo < 2; ++eo) it_half<R>(ch, cst, eo, part, flags, 0, nh, 0, s);
+  gf_check(ch, cst, part, nh, 1, s);
 }
 
 template <typename R>
@@ -411,22 +514,22 @@ void launch_sum_partials(const double* part, int nblocks, int nq, double* out, c
   else sum_partials_kernel<4><<<1, 1024, 0, s>>>(part, nblocks, out);
 }
 
-template void launch_gf_iteration<float>(const ChainDev*, ChainState*, int, double*, int, cudaStream_t);
-template void launch_gf_iteration<double>(const ChainDev*, ChainState*, int, double*, int, cudaStream_t);
+template void launch_gf_batch<float>(const ChainDev*, ChainState*, int, int, double*, int, int, cudaStream_t);
+template void launch_gf_batch<double>(const ChainDev*, ChainState*, int, int, double*, int, int, cudaStream_t);
 template int launch_gf_half<float>(const ChainDev*, ChainState*, int, int, double*, int, int, int, cudaStream_t);
 template int launch_gf_half<double>(const ChainDev*, ChainState*, int, int, double*, int, int, int, cudaStream_t);
 template <typename R>
 int launch_it_half(const ChainDev* ch, ChainState* cst, int eo, int last, double* part, int nh, int s_lo, int flags,
                    cudaStream_t s) {
   const int nb = ceil_div(nh - 2 * s_lo, kBlock);
-  (void)launch_pdl(it_half_kernel<R>, nb, kBlock, 0, s, ch, (const ChainState*)cst, eo, part, flags, 1, s_lo, last);
+  (void)launch_pdl(it_half_kernel<R, kBlock>, nb, kBlock, 0, s, ch, cst, eo, part, flags, 1, s_lo, last, 0);
   return nb;
 }
 template int launch_it_half<float>(const ChainDev*, ChainState*, int, int, double*, int, int, int, cudaStream_t);
 template int launch_it_half<double>(const ChainDev*, ChainState*, int, int, double*, int, int, int, cudaStream_t);
 
-template void launch_it_iteration<float>(const ChainDev*, ChainState*, int, int, double*, int, cudaStream_t);
-template void launch_it_iteration<double>(const ChainDev*, ChainState*, int, int, double*, int, cudaStream_t);
+template void launch_it_iteration<float>(const ChainDev*, ChainState*, int, double*, int, cudaStream_t);
+template void launch_it_iteration<double>(const ChainDev*, ChainState*, int, double*, int, cudaStream_t);
 template int launch_gf_theta<float>(const ChainDev*, double*, int, cudaStream_t);
 template int launch_gf_theta<double>(const ChainDev*, double*, int, cudaStream_t);
 

@@ -171,10 +171,8 @@ struct PassArgs {
   // programmatic dependent launch of the per-pass kernels.  rng_early: draw
   // the first site's uniforms before griddepcontrol.wait (the RNG counters,
   // written only by the finalize kernel, are settled for every pass but the
-  // first of a queue).  trigger_late: let dependents launch only after this
-  // kernel's wait (the first pass of a queue, so that no later pass can read
-  // the counters while an earlier finalize still writes them).
-  int rng_early, trigger_late;
+  // first of a queue: the later ones launch after its wait).
+  int rng_early;
   // reduce-behind: blocks [ntiles, gridDim.x) of a per-pass launch sum the
   // previous pass's tile partials (slot rb_slot & 0xff, tile table rb_slot >>
   // 8; the buffers in *st) into level-1 chunk sums (lce_update.cu), the same
@@ -290,9 +288,12 @@ void launch_init_hot(void* u, void* a, int nh, uint32_t k0, uint32_t k1, cudaStr
 void launch_flush(void* buf, size_t bytes, cudaStream_t s);
 
 // ---- gauge fixing (lce_gaugefix.cu)
+// n iterations of a fixing with their checks: the overrelaxed form (track: also
+// the transform G), or with it_flags >= 0 f/it_gauge_fixing.f (flags
+// LCE_ITGF_*, step from cst->gf_step) with reunitarisation
 template <typename R>
-void launch_gf_iteration(const ChainDev* ch, ChainState* cst, int track, double* part, int nh,
-                         cudaStream_t s);
+void launch_gf_batch(const ChainDev* ch, ChainState* cst, int track, int it_flags, double* part, int nh, int n,
+                     cudaStream_t s);
 // one overrelaxed half-step over sites [s_lo, nh - s_lo) of local parity eo
 // (a z-slab: s_lo = one plane); last: the second half-step, which writes the
 // theta partials into part and reunitarises; track: also accumulate the
@@ -309,11 +310,10 @@ int launch_it_half(const ChainDev* ch, ChainState* cst, int eo, int last, double
 // convergence test of a z-slab decomposed fixing from the slabs' theta sums
 void launch_gf_check_slabs(const ChainDev* ch, ChainState* cst, const double* sums, int nslabs, double nh,
                            cudaStream_t s, int fa = 0);
-// one iteration of f/it_gauge_fixing.f (flags LCE_ITGF_*, step from cst->gf_step),
-// then the convergence check of the overrelaxed form
+// one iteration of f/it_gauge_fixing.f as the subroutine leaves it (no
+// reunitarisation), then the convergence check of the overrelaxed form
 template <typename R>
-void launch_it_iteration(const ChainDev* ch, ChainState* cst, int flags, int renorm, double* part, int nh,
-                         cudaStream_t s);
+void launch_it_iteration(const ChainDev* ch, ChainState* cst, int flags, double* part, int nh, cudaStream_t s);
 template <typename R>
 void launch_gauge_apply(const ChainDev* ch, int nh, cudaStream_t s);
 template <typename R>
