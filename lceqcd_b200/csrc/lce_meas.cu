@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kCorrThreads) correlators_kernel(const double*
 }
 
 // plaquette 1/2 Re Tr U_mu(x) U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+ over both
-// parities, each link read from HBM once (256^3 FP32: 199 us, 283 us with one
+// parities, each link read from HBM once (256^3 FP32: 210 us, 283 us with one
 // parity after the other).  A block sums several tiles, at most kSumBlocks
 // blocks in all, so that their partial sums are few.
 template <typename R>
@@ -177,18 +177,16 @@ __global__ void __launch_bounds__(kBlock) plaquette_kernel(const ChainDev* chp, 
     const int oe = 1 - eo;
     const Coord X = site_coord(eo, s, ch.hx, ch.nxy, ch.dhx, ch.dnxy);
     const NbrOff o = nbr_offsets(ch, X);
-    su2<R> u[3], w[3][3];  // U_mu(x); w[mu][nu] = U_mu(x + nu), nu != mu
-#pragma unroll
-    for (int mu = 0; mu < 3; ++mu) {
-      u[mu] = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + eo)) * nh + s);
-#pragma unroll
-      for (int nu = 0; nu < 3; ++nu)
-        if (nu != mu) w[mu][nu] = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + oe)) * nh + (s + o.p[nu]));
-    }
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu)
 #pragma unroll
-      for (int nu = mu + 1; nu < 3; ++nu) v[0] += (double)nn(nn(u[mu], w[nu][mu]), dd(w[mu][nu], u[nu])).a.re;
+      for (int nu = mu + 1; nu < 3; ++nu) {
+        const su2<R> p = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + eo)) * nh + s);
+        const su2<R> q = LinkIO<R>::ld(ch.u, ((size_t)(nu * 2 + oe)) * nh + (s + o.p[mu]));
+        const su2<R> t = LinkIO<R>::ld(ch.u, ((size_t)(mu * 2 + oe)) * nh + (s + o.p[nu]));
+        const su2<R> e = LinkIO<R>::ld(ch.u, ((size_t)(nu * 2 + eo)) * nh + s);
+        v[0] += (double)nn(nn(p, q), dd(t, e)).a.re;
+      }
   }
   block_reduce_store<1>(v, part + blockIdx.x);
 }
