@@ -878,8 +878,12 @@ __global__ void __launch_bounds__(kBlock) fa_exp_apply_kernel(FaArgs a, int l0, 
   }
   __syncthreads();
   if (i >= nm) return;
+  // g as new values: the FP64 products of values the compiler knows to come
+  // from here were contracted otherwise than fa_apply_kernel's
   auto g_at = [&](int p) {
-    return su2<double>{{fa_gs[p], fa_gs[np + p]}, {fa_gs[2 * np + p], fa_gs[3 * np + p]}};
+    su2<double> g{{fa_gs[p], fa_gs[np + p]}, {fa_gs[2 * np + p], fa_gs[3 * np + p]}};
+    asm volatile("" : "+d"(g.a.re), "+d"(g.a.im), "+d"(g.b.re), "+d"(g.b.im));
+    return g;
   };
   const int up[3] = {xx + 1 < S ? i + 1 : hx0 + zz * T + yy, yy + 1 < T ? i + S : hy0 + zz * S + xx,
                      zz + 1 < U ? i + S * T : hz0 + yy * S + xx};
