@@ -70,8 +70,8 @@ extern "C" {
  * CUDA graph (one site per thread, or two sites per thread), or one
  * cooperative persistent kernel per sweep that loops over the (chain, tile)
  * work list of every pass with a grid barrier in between.  AUTO times the
- * forms -- and, for FP32 contexts, the tile shapes of the per-pass forms
- * (128, 256, 448 or 512 threads per block, see lce_params.tile_threads) -- on the
+ * forms -- and the tile shapes of the per-pass forms (128, 256, 448 or 512
+ * threads per block, in FP64 128 or 256, see lce_params.tile_threads) -- on the
  * first sweeps and keeps the fastest (lce_get_sweep_mode, lce_get_tile_shape). */
 #define LCE_SWEEP_AUTO 0
 #define LCE_SWEEP_PASSES 1
@@ -118,7 +118,8 @@ typedef struct lce_params {
                             0 (default) = tuned with LCE_SWEEP_AUTO, else 256;
                             or 128, 256, 448, 512 (448: one site per thread
                             only).  FP32 only: the FP64 validation
-                            path and z-slabs use 256.  Results do not depend on
+                            path uses 256 (0 with LCE_SWEEP_AUTO: tuned,
+                            128 or 256) and z-slabs 256.  Results do not depend on
                             it (per-site work and random numbers are the same;
                             FP64 sums are grouped per tile). */
   int tile_registers;    /* per-thread register cap of those kernels: 0

@@ -575,7 +575,7 @@ constexpr size_t kTuneSamples = 3;
 bool sweeps_defer_finalize(const lce_ctx* c, int form, int bs, int spt, int occ) {
   if (form != LCE_SWEEP_PASSES || spt != 1 || occ != 0 || c->nchains != 1) return false;
   if (c->chunks[tile_index(bs, spt)].back() > 8) return false;
-  return c->prec == LCE_PREC_F64 ? bs == 256 : (bs == 128 || bs == 256 || bs == 448 || bs == 512);
+  return c->prec == LCE_PREC_F64 ? (bs == 128 || bs == 256) : (bs == 128 || bs == 256 || bs == 448 || bs == 512);
 }
 
 // nrep sweeps with deferred finalizes: sweep r's passes take the RNG offsets
@@ -936,9 +936,10 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
     return nullptr;
   }
   // tile shape: FP32 contexts tune threads per block (128, 256, 512) and sites
-  // per thread under AUTO unless tile_threads fixes the block; the FP64
-  // validation path and z-slabs use kBlock threads
-  c->tile_req = (c->prec == LCE_PREC_F32 && !slab) ? p[0].tile_threads : kBlock;
+  // per thread under AUTO unless tile_threads fixes the block; FP64 contexts
+  // tune 128 or kBlock threads under AUTO if tile_threads leaves it open, and
+  // use kBlock otherwise, as z-slabs do
+  c->tile_req = !slab && (c->prec == LCE_PREC_F32 || p[0].tile_threads == 0) ? p[0].tile_threads : kBlock;
   c->tile_bs = c->tile_req ? c->tile_req : kBlock;
   c->tile_spt = c->mode == LCE_SWEEP_PASSES2 ? 2 : 1;
   if (c->tile_spt == 2 && c->tile_bs > 256) c->tile_bs = kBlock;  // (448, 2), (512, 2) are not compiled
@@ -956,9 +957,9 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
         break;
       }
       if (c->tile_req && b != c->tile_req) continue;
-      if (c->prec == LCE_PREC_F64 && b != kBlock) continue;
+      if (c->prec == LCE_PREC_F64 && b > kBlock) continue;
       c->tune.push_back(TuneForm{LCE_SWEEP_PASSES, b, 1, 0, {}});
-      if (b <= 256) c->tune.push_back(TuneForm{LCE_SWEEP_PASSES2, b, 2, 0, {}});
+      if (b <= 256 && !(c->prec == LCE_PREC_F64 && b == 128)) c->tune.push_back(TuneForm{LCE_SWEEP_PASSES2, b, 2, 0, {}});
     }
     // Not candidates, measured slower on the B200 at 64^3 and 128^3 (still
     // selectable): the 56-register 128-thread form (tile_registers = 56,

@@ -1092,8 +1092,12 @@ void launch_link_t(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStr
 
 // Tile shapes compiled: FP32 (BS, SPT) in {128, 256, 512} x {1} and
 // {128, 256} x {2} at the 64-register cap, (448, 1) at two blocks per SM (72
-// registers), and (128, 1) at 56 registers (a.occ = 1152); the FP64
-// validation path only BS = 256.
+// registers), and (128, 1) at 56 registers (a.occ = 1152); FP64 (256, 1),
+// (256, 2) and (128, 1).  FP64 with 128 instead of 256 threads, us per sweep
+// with measurements: 8^3 36.1 -> 32.6 and 24^3 41.0 -> 38.2 (few blocks: a
+// pass is the latency of the SM with the most warps), 32^3 41.6 -> 41.5, 48^3
+// 63.8 -> 66.1, 64^3 96.6 -> 94.6 (a finer last wave); a looser register cap
+// (128) changed nothing.  The autotuner tells them apart.
 template <typename R>
 void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
@@ -1101,9 +1105,8 @@ void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) 
       launch_higgs_t<R, 1, 128, 1152>(mode, a, nblocks, s);
       return;
     }
-    if (a.bs == 128) {
-      if (a.spt == 2) launch_higgs_t<R, 2, 128>(mode, a, nblocks, s);
-      else launch_higgs_t<R, 1, 128>(mode, a, nblocks, s);
+    if (a.bs == 128 && a.spt == 2) {
+      launch_higgs_t<R, 2, 128>(mode, a, nblocks, s);
       return;
     }
     if (a.bs == 512) {
@@ -1115,7 +1118,8 @@ void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) 
       return;
     }
   }
-  if (a.spt == 2) launch_higgs_t<R, 2, 256>(mode, a, nblocks, s);
+  if (a.bs == 128) launch_higgs_t<R, 1, 128>(mode, a, nblocks, s);
+  else if (a.spt == 2) launch_higgs_t<R, 2, 256>(mode, a, nblocks, s);
   else launch_higgs_t<R, 1, 256>(mode, a, nblocks, s);
 }
 
@@ -1126,9 +1130,8 @@ void launch_link(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStrea
       launch_link_t<R, 1, 128, 1152>(mode, mu, a, nblocks, s);
       return;
     }
-    if (a.bs == 128) {
-      if (a.spt == 2) launch_link_t<R, 2, 128>(mode, mu, a, nblocks, s);
-      else launch_link_t<R, 1, 128>(mode, mu, a, nblocks, s);
+    if (a.bs == 128 && a.spt == 2) {
+      launch_link_t<R, 2, 128>(mode, mu, a, nblocks, s);
       return;
     }
     if (a.bs == 512) {
@@ -1140,19 +1143,16 @@ void launch_link(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStrea
       return;
     }
   }
-  if (a.spt == 2) launch_link_t<R, 2, 256>(mode, mu, a, nblocks, s);
+  if (a.bs == 128) launch_link_t<R, 1, 128>(mode, mu, a, nblocks, s);
+  else if (a.spt == 2) launch_link_t<R, 2, 256>(mode, mu, a, nblocks, s);
   else launch_link_t<R, 1, 256>(mode, mu, a, nblocks, s);
 }
 
 // the first pass of a sweep carrying the previous sweep's finalize (one site
-// per thread, 128 (64 registers), 256, 448 or 512 threads in FP32; 256 in FP64)
+// per thread, 128 (64 registers in FP32) or 256 threads, in FP32 also 448 or 512)
 template <typename R>
 void launch_higgs_fin(const PassArgsMany& a, const FinalizeArgs& fp, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
-    if (a.bs == 128) {
-      (void)launch_pdl(higgs_fin_kernel<R, 128>, nblocks, 128, 0, s, one_of(a), fp);
-      return;
-    }
     if (a.bs == 448) {
       (void)launch_pdl(higgs_fin_kernel<R, 448>, nblocks, 448, 0, s, one_of(a), fp);
       return;
@@ -1162,7 +1162,8 @@ void launch_higgs_fin(const PassArgsMany& a, const FinalizeArgs& fp, int nblocks
       return;
     }
   }
-  (void)launch_pdl(higgs_fin_kernel<R, 256>, nblocks, 256, 0, s, one_of(a), fp);
+  if (a.bs == 128) (void)launch_pdl(higgs_fin_kernel<R, 128>, nblocks, 128, 0, s, one_of(a), fp);
+  else (void)launch_pdl(higgs_fin_kernel<R, 256>, nblocks, 256, 0, s, one_of(a), fp);
 }
 template void launch_higgs_fin<float>(const PassArgsMany&, const FinalizeArgs&, int, cudaStream_t);
 template void launch_higgs_fin<double>(const PassArgsMany&, const FinalizeArgs&, int, cudaStream_t);
