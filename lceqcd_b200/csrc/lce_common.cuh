@@ -292,9 +292,10 @@ struct Uniforms {
 // Programmatic dependent launch (sm_90+): a kernel lets the next kernel of
 // its stream begin launching once every block of it has started, and the
 // next kernel blocks in griddepcontrol.wait until this grid has completed
-// and its writes are visible.  Kernels call pdl_trigger() first, do
-// data-independent set-up, and call pdl_wait() before their first read of
-// anything an earlier kernel writes.
+// and its writes are visible.  Kernels do data-independent set-up, call
+// pdl_wait() before their first read of anything an earlier kernel writes,
+// and pdl_trigger() right after it (one-block kernels at their start): with
+// the trigger first, the blocks of several waiting kernels fill the SMs.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

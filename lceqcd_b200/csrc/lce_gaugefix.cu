@@ -11,11 +11,13 @@
 // Every link touched in a half-step belongs to exactly one thread, so the
 // update is race free.  All links are rewritten in the eo = 1 half-step, so
 // reunitarising there is exactly f/u_f_renorm.f after the iteration
-// (f/landau_gauge.f:54-59).  A one-block check kernel sums the partials in a
-// fixed order, counts the iteration and raises a device flag when theta <=
-// limit_or (or the cap is reached); later kernels of a captured batch of
-// iterations see the flag and return at once, so the host reads the state
-// only once per batch.
+// (f/landau_gauge.f:54-59).  The check sums the partials in a fixed order,
+// counts the iteration and raises a device flag when theta <= limit_or (or
+// the cap is reached): a one-block kernel after each iteration, or, while a
+// block can add the partials itself (kGfMaxPartials), the blocks of the next
+// half-step, with the kernel only at a batch's end.  Later kernels of a
+// captured batch see the flag and return at once, so the host reads the
+// state only once per batch.
 #include <algorithm>
 
 #include "lce_internal.hpp"
