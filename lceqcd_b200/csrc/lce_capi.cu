@@ -237,9 +237,14 @@ const lce_meas* report_meas(const lce_ctx* c) {
   return reinterpret_cast<const lce_meas*>(reinterpret_cast<const char*>(c->report.data()) + kReportState);
 }
 
-int status_check(lce_ctx* c) {
+int report_read(lce_ctx* c) {
   CK(cudaMemcpyAsync(c->report.data(), c->st_d, report_bytes(c), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  return LCE_OK;
+}
+
+// the error that the state read last reports
+int report_status(lce_ctx* c) {
   const CtxState& st = *reinterpret_cast<const CtxState*>(c->report.data());
   if (st.status) {
     unsigned int z = 0;
@@ -253,6 +258,11 @@ int status_check(lce_ctx* c) {
     return fail(c, LCE_ERR_NAN, "non-finite value in a measurement reduction");
   }
   return LCE_OK;
+}
+
+int status_check(lce_ctx* c) {
+  const int rc = report_read(c);
+  return rc ? rc : report_status(c);
 }
 
 int nslots_of(unsigned char kind) {
@@ -2266,17 +2276,17 @@ int lce_sweep(lce_ctx* c, int measflag, lce_meas* m) {
 int lce_get_meas(lce_ctx* c, int chain, lce_meas* m) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !m || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
-  const int rc = status_check(c);
+  if (const int rc = report_read(c)) return rc;
   *m = report_meas(c)[chain];
-  return rc;
+  return report_status(c);
 }
 
 int lce_get_meas_batch(lce_ctx* c, lce_meas* m) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !m) return LCE_ERR_INVALID;
-  const int rc = status_check(c);
+  if (const int rc = report_read(c)) return rc;
   std::copy(report_meas(c), report_meas(c) + c->nchains, m);
-  return rc;
+  return report_status(c);
 }
 
 int lce_landau_gauge(lce_ctx* c, int chain, double* theta, int* iters, int max_iters) {
