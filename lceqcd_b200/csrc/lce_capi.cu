@@ -224,21 +224,24 @@ bool valid_params(const lce_params& p, std::string& why) {
   return true;
 }
 
-// The state and every chain's last measurements, copied to the host in one
-// piece behind the work queued so far: one copy and one synchronisation where
-// a read of the status and a read of the measurements were two of each (a
-// measured 16^3 FP64 sweep with its values read back 156 -> 146 us).  Pageable
-// memory: pinning a page takes ~3 ms of a context's creation, and the copy is a
-// few hundred bytes.
+// The state and the last measurements of the first nrec chains, copied to the
+// host in one piece behind the work queued so far: one copy and one
+// synchronisation where a read of the status and a read of the measurements
+// were two of each (a measured 16^3 FP64 sweep with its values read back 156 ->
+// 146 us).  nrec is 0 for the state alone, 1 for a single chain's values and
+// the acceptances, and every chain only where every chain's are returned: the
+// records of a large batch on each read would make a loop over its chains
+// quadratic.  Pageable memory: pinning a page takes ~3 ms of a context's
+// creation, and the copy is a few hundred bytes.
 constexpr size_t kReportState = 256;
 static_assert(sizeof(CtxState) <= kReportState, "the measurements follow the state");
-size_t report_bytes(const lce_ctx* c) { return kReportState + sizeof(lce_meas) * c->nchains; }
-const lce_meas* report_meas(const lce_ctx* c) {
-  return reinterpret_cast<const lce_meas*>(reinterpret_cast<const char*>(c->report.data()) + kReportState);
+size_t report_bytes(int nrec) { return kReportState + sizeof(lce_meas) * nrec; }
+lce_meas* report_meas(lce_ctx* c) {
+  return reinterpret_cast<lce_meas*>(reinterpret_cast<char*>(c->report.data()) + kReportState);
 }
 
-int report_read(lce_ctx* c) {
-  CK(cudaMemcpyAsync(c->report.data(), c->st_d, report_bytes(c), cudaMemcpyDeviceToHost, c->stream));
+int report_read(lce_ctx* c, int nrec) {
+  CK(cudaMemcpyAsync(c->report.data(), c->st_d, report_bytes(nrec), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return LCE_OK;
 }
@@ -260,8 +263,8 @@ int report_status(lce_ctx* c) {
   return LCE_OK;
 }
 
-int status_check(lce_ctx* c) {
-  const int rc = report_read(c);
+int status_check(lce_ctx* c, int nrec = 0) {
+  const int rc = report_read(c, nrec);
   return rc ? rc : report_status(c);
 }
 
@@ -676,7 +679,7 @@ int routine_call(lce_ctx* c, unsigned char kind, int measflag, float* accept, bo
   int rc = enqueue(c, {kind}, measflag, renorm);
   if (rc) return rc;
   if (!accept) return LCE_OK;
-  rc = status_check(c);
+  rc = status_check(c, 1);
   if (rc) return rc;
   const lce_meas& m = *report_meas(c);
   switch (kind) {
@@ -920,10 +923,10 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
     if ((e = cudaMalloc(&c->chunks_d, sizeof(double) * nd)) != cudaSuccess) return bail(e, "cudaMalloc(chunk sums)");
   }
   c->blk_d = c->tiles_d[1];
-  if ((e = cudaMalloc(&c->st_d, report_bytes(c))) != cudaSuccess) return bail(e, "cudaMalloc(state)");
-  if ((e = cudaMemset(c->st_d, 0, report_bytes(c))) != cudaSuccess) return bail(e, "cudaMemset(state)");
+  if ((e = cudaMalloc(&c->st_d, report_bytes(n))) != cudaSuccess) return bail(e, "cudaMalloc(state)");
+  if ((e = cudaMemset(c->st_d, 0, report_bytes(n))) != cudaSuccess) return bail(e, "cudaMemset(state)");
   c->meas_d = reinterpret_cast<lce_meas*>(reinterpret_cast<char*>(c->st_d) + kReportState);
-  c->report.assign((report_bytes(c) + sizeof(double) - 1) / sizeof(double), 0.0);
+  c->report.assign((report_bytes(n) + sizeof(double) - 1) / sizeof(double), 0.0);
   c->delta_h.assign(n, 0.0);
   if ((e = cudaMalloc(&c->cst_d, sizeof(ChainState) * n)) != cudaSuccess) return bail(e, "cudaMalloc(cstate)");
   {
@@ -2276,7 +2279,10 @@ int lce_sweep(lce_ctx* c, int measflag, lce_meas* m) {
 int lce_get_meas(lce_ctx* c, int chain, lce_meas* m) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !m || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
-  if (const int rc = report_read(c)) return rc;
+  // chain 0's record follows the state; another chain's is a copy of its own
+  if (chain > 0)
+    CK(cudaMemcpyAsync(report_meas(c) + chain, c->meas_d + chain, sizeof(*m), cudaMemcpyDeviceToHost, c->stream));
+  if (const int rc = report_read(c, chain > 0 ? 0 : 1)) return rc;
   *m = report_meas(c)[chain];
   return report_status(c);
 }
@@ -2284,7 +2290,7 @@ int lce_get_meas(lce_ctx* c, int chain, lce_meas* m) {
 int lce_get_meas_batch(lce_ctx* c, lce_meas* m) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !m) return LCE_ERR_INVALID;
-  if (const int rc = report_read(c)) return rc;
+  if (const int rc = report_read(c, c->nchains)) return rc;
   std::copy(report_meas(c), report_meas(c) + c->nchains, m);
   return report_status(c);
 }

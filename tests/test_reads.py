@@ -57,3 +57,29 @@ assert lib.lce_get_meas(c, 2, C.byref(m)) == 0 and bytes(m) == bytes(REC)
 assert lib.lce_get_meas_batch(c, b) == 0 and bytes(b) == bytes(3 * REC)
 lib.lce_destroy(c)
 """)
+
+
+@pytest.mark.parametrize("n", [1, 3, 1000])
+def test_a_read_copies_what_it_returns(fake, n):
+    """The state and the record asked for, not every chain's: a loop over the
+    chains stays linear in their number.  A single chain's values and the last
+    call's acceptance take one copy."""
+    fake(f"""
+n = {n}
+c = create(n)
+m, b, f = _lib.LceMeas(), (_lib.LceMeas * n)(), C.c_float(0.5)
+def cost(call):
+    fake.fake_reset(0, 0)
+    assert call() == 0
+    return fake.fake_d2h_bytes(), fake.fake_d2h_copies()
+STATE = 256
+assert cost(lambda: lib.lce_synchronize(c)) <= (STATE, 1)
+for chain in {{0, n // 2, n - 1}}:
+    size, copies = cost(lambda: lib.lce_get_meas(c, chain, C.byref(m)))
+    assert size <= STATE + REC and copies <= (1 if chain == 0 else 2), (chain, size, copies)
+for call in (lambda: lib.lce_ahiggs2(c, 1, C.byref(f)), lambda: lib.lce_ahiggs1(c, C.byref(f), 1, None)):
+    size, copies = cost(call)
+    assert size <= STATE + REC and copies == 1, (size, copies)
+assert cost(lambda: lib.lce_get_meas_batch(c, b)) == (STATE + n * REC, 1)
+lib.lce_destroy(c)
+""")
