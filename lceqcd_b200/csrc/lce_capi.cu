@@ -43,7 +43,8 @@ void lce::set_thread_error(const std::string& msg) { g_create_error = msg; }
 // shape (threads per block, sites per thread), with its timed samples
 struct TuneForm {
   int form, bs, spt, occ;  // occ: resident threads per SM of the register cap (0: the default)
-  std::vector<float> ms;
+  std::vector<float> ms;   // per sweep, of each timed run
+  int sweeps;              // run so far, the discarded first one included
 };
 
 struct lce_ctx {
@@ -122,6 +123,7 @@ struct lce_ctx {
   int tile_bs = kBlock, tile_spt = 1;  // tile shape of the per-pass kernels in use
   int tile_occ = 0;                    // its register-cap occupancy (0: the default)
   std::vector<TuneForm> tune;        // autotune candidates and their samples
+  std::vector<cudaEvent_t> tune_ev;  // the events between the runs of a tuning call
   std::map<std::pair<int, int>, cudaGraphExec_t> gf_exec;
   std::string err;
 };
@@ -579,7 +581,7 @@ int enqueue_persistent(lce_ctx* c, const std::vector<unsigned char>& routines, i
   return LCE_OK;
 }
 
-constexpr size_t kTuneSamples = 3;
+constexpr int kTuneSweeps = 4;
 
 // Graphs of several sweeps defer each sweep's finalize (but the last) into an
 // extra block of the next sweep's first pass (higgs_fin_kernel): a single
@@ -673,6 +675,80 @@ std::vector<unsigned char> sweep_routines(const lce_ctx* c) {
   r.push_back(c->agauge_hits == 3 ? kLinkHB3 : kLinkHB);
   for (int i = 0; i < c->n_link_or; ++i) r.push_back(kLinkOR);
   return r;
+}
+
+// Autotune on real sweeps: each candidate (sweep form and tile shape) runs one
+// discarded sweep and kTuneSweeps timed ones, and the fastest is kept.  The
+// timed sweeps of a candidate are replayed back to back between two events, the
+// candidates' runs queued behind one another.  Events around a single sweep, with
+// a synchronisation after each, also timed the host's launch of its graph (8 us,
+// +- 1.5 us), and events on a busy stream come in steps of 2.05 us, so in either
+// way shapes a few percent apart were taken for one another.  Of 24 fresh
+// contexts the faster shape now goes to 20 at 32^3 in FP32 (28.6 against 30.8 us
+// per sweep; 10 with the median of three single sweeps), to 24 at 24^3 (27.0,
+// 28.4; 21), and in FP64 to 24 at 56^3 (70.9, 72.2; 23) as at 48^3 and 64^3.  A
+// call's first sweep, behind an idle stream, is not timed unless every sweep is a
+// call of its own.  Adds the sweeps queued to *done.
+int tune_sweeps(lce_ctx* c, int nsweeps, int mf, int* done) {
+  struct Run {
+    int form, sweeps;  // form -1: not timed
+  };
+  std::vector<Run> runs;
+  std::vector<int> had;  // each candidate's sweeps, the discarded one included
+  for (const TuneForm& f : c->tune) had.push_back(f.sweeps);
+  while (*done < nsweeps) {
+    auto next = std::find(had.begin(), had.end(), 0);
+    if (next == had.end()) next = std::find_if(had.begin(), had.end(), [](int n) { return n <= kTuneSweeps; });
+    if (next == had.end()) break;
+    const int k = (int)(next - had.begin()), left = nsweeps - *done;
+    const TuneForm tf = c->tune[k];
+    cudaGraphExec_t ex = nullptr;
+    if (tf.form != LCE_SWEEP_DIRECT) {
+      if (int rc = sweep_graph(c, tf.form, tf.bs, tf.spt, tf.occ, mf, &ex)) return rc;
+      if (c->mode != LCE_SWEEP_AUTO) return LCE_OK;  // the persistent form was unavailable
+    }
+    while (c->tune_ev.size() < runs.size() + 2) {
+      cudaEvent_t e;
+      CK(cudaEventCreate(&e));
+      c->tune_ev.push_back(e);
+    }
+    const bool idle = *next > 0 && runs.empty() && left > 1;
+    const int m = *next == 0 || idle ? 1 : std::min(left, 1 + kTuneSweeps - *next);
+    if (runs.empty()) CK(cudaEventRecord(c->tune_ev[0], c->stream));
+    for (int i = 0; i < m; ++i) {
+      if (ex) CK(cudaGraphLaunch(ex, c->stream));
+      else if (int rc = enqueue(c, sweep_routines(c), mf, true, nullptr, tf.bs, tf.spt, tf.occ)) return rc;
+    }
+    CK(cudaEventRecord(c->tune_ev[runs.size() + 1], c->stream));
+    runs.push_back(Run{*next == 0 || idle ? -1 : k, m});
+    if (!idle) *next += m;
+    *done += m;
+  }
+  if (runs.empty()) return LCE_OK;
+  CK(cudaEventSynchronize(c->tune_ev[runs.size()]));
+  for (size_t i = 0; i < runs.size(); ++i) {
+    float ms = 0;
+    CK(cudaEventElapsedTime(&ms, c->tune_ev[i], c->tune_ev[i + 1]));
+    if (runs[i].form >= 0) c->tune[runs[i].form].ms.push_back(ms / runs[i].sweeps);
+  }
+  for (size_t f = 0; f < had.size(); ++f) c->tune[f].sweeps = had[f];
+  if (*std::min_element(had.begin(), had.end()) <= kTuneSweeps) return LCE_OK;
+  int best = 0;
+  float best_med = 0;
+  for (int f = 0; f < (int)c->tune.size(); ++f) {
+    std::vector<float> v(c->tune[f].ms);
+    std::sort(v.begin(), v.end());
+    const float med = v[v.size() / 2];
+    if (f == 0 || med < best_med) {
+      best = f;
+      best_med = med;
+    }
+  }
+  c->mode = c->tune[best].form;
+  c->tile_bs = c->tune[best].bs;
+  c->tile_spt = c->tune[best].spt;
+  c->tile_occ = c->tune[best].occ;
+  return LCE_OK;
 }
 
 int routine_call(lce_ctx* c, unsigned char kind, int measflag, float* accept, bool renorm) {
@@ -966,20 +1042,20 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
     const int bss[4] = {128, 256, 448, 512};
     for (int b : bss) {
       if (reg56) {
-        c->tune.push_back(TuneForm{LCE_SWEEP_PASSES, 128, 1, 1152, {}});
+        c->tune.push_back(TuneForm{LCE_SWEEP_PASSES, 128, 1, 1152, {}, 0});
         break;
       }
       if (c->tile_req && b != c->tile_req) continue;
       if (c->prec == LCE_PREC_F64 && b > kBlock) continue;
-      c->tune.push_back(TuneForm{LCE_SWEEP_PASSES, b, 1, 0, {}});
-      if (b <= 256 && !(c->prec == LCE_PREC_F64 && b == 128)) c->tune.push_back(TuneForm{LCE_SWEEP_PASSES2, b, 2, 0, {}});
+      c->tune.push_back(TuneForm{LCE_SWEEP_PASSES, b, 1, 0, {}, 0});
+      if (b <= 256 && !(c->prec == LCE_PREC_F64 && b == 128)) c->tune.push_back(TuneForm{LCE_SWEEP_PASSES2, b, 2, 0, {}, 0});
     }
     // Not candidates, measured slower on the B200 at 64^3 and 128^3 (still
     // selectable): the 56-register 128-thread form (tile_registers = 56,
     // 71.1 / 381.1 us per sweep against 64.7 / 374-377 us) and the direct
     // launches without a graph (LCE_SWEEP_DIRECT, 66.0 / 380.0 us against
     // 64.6 / 377.5 us with the same tile).
-    if (c->persist_grid > 0) c->tune.push_back(TuneForm{LCE_SWEEP_PERSISTENT, kBlock, 1, 0, {}});
+    if (c->persist_grid > 0) c->tune.push_back(TuneForm{LCE_SWEEP_PERSISTENT, kBlock, 1, 0, {}, 0});
   }
   c->part_slots = std::max(6, 4 + 6 + 2 * c->n_higgs_metro + 6 * c->n_link_or);
   c->slot_stride = (size_t)c->tiles[0].back() * kNQ;  // the most tiles: 128 sites each
@@ -1936,6 +2012,7 @@ void lce_destroy(lce_ctx* c) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->prof_ev) cudaEventDestroy(e);
+  for (cudaEvent_t e : c->tune_ev) cudaEventDestroy(e);
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->side) cudaStreamDestroy(c->side);
@@ -2187,49 +2264,8 @@ int lce_sweeps(lce_ctx* c, int nsweeps, int measflag) {
   if (!c || nsweeps < 0) return LCE_ERR_INVALID;
   const int mf = measflag == 1 ? 1 : 0;
   int done = 0;
-  // autotune: rotate through the candidates (sweep forms and tile shapes) on
-  // real sweeps, one timed sweep at a time, until each has kTuneSamples
-  // samples after a discarded first one; then keep the fastest by median.
-  while (c->mode == LCE_SWEEP_AUTO && done < nsweeps) {
-    int k = 0;
-    for (int f = 1; f < (int)c->tune.size(); ++f)
-      if (c->tune[f].ms.size() < c->tune[k].ms.size()) k = f;
-    const TuneForm tf = c->tune[k];
-    cudaGraphExec_t ex = nullptr;
-    if (tf.form != LCE_SWEEP_DIRECT) {
-      int rc = sweep_graph(c, tf.form, tf.bs, tf.spt, tf.occ, mf, &ex);
-      if (rc) return rc;
-      if (c->mode != LCE_SWEEP_AUTO) break;  // the persistent form was unavailable
-    }
-    CK(cudaEventRecord(c->ev0, c->stream));
-    if (ex) CK(cudaGraphLaunch(ex, c->stream));
-    else if (int rc = enqueue(c, sweep_routines(c), mf, true, nullptr, tf.bs, tf.spt, tf.occ)) return rc;
-    CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->tune[k].ms.push_back(ms);
-    ++done;
-    bool complete = true;
-    for (const TuneForm& f : c->tune) complete = complete && f.ms.size() >= kTuneSamples + 1;
-    if (complete) {
-      int best = 0;
-      float best_med = 0;
-      for (int f = 0; f < (int)c->tune.size(); ++f) {
-        std::vector<float> v(c->tune[f].ms.begin() + 1, c->tune[f].ms.end());
-        std::sort(v.begin(), v.end());
-        const float med = v[v.size() / 2];
-        if (f == 0 || med < best_med) {
-          best = f;
-          best_med = med;
-        }
-      }
-      c->mode = c->tune[best].form;
-      c->tile_bs = c->tune[best].bs;
-      c->tile_spt = c->tune[best].spt;
-      c->tile_occ = c->tune[best].occ;
-    }
-  }
+  if (c->mode == LCE_SWEEP_AUTO)
+    if (int rc = tune_sweeps(c, nsweeps, mf, &done)) return rc;
   if (done < nsweeps) {
     if (c->mode == LCE_SWEEP_DIRECT) {
       const std::vector<unsigned char> r = sweep_routines(c);

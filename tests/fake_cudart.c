@@ -1,7 +1,10 @@
 /* A CUDA runtime in host memory for tests without a GPU: preloaded before
- * libcudart, it replaces the calls that a context's creation and its reads of
- * values make.  Kernels do not run.  It counts the bytes copied to the host
- * and can refuse those copies or the synchronisation after them. */
+ * libcudart, it replaces the calls that a context's creation, its sweeps and
+ * its reads of values make.  Kernels do not run.  It counts the bytes copied to
+ * the host and can refuse those copies or the synchronisation after them.  Time
+ * is a model: a host clock that calls advance, a device clock that kernels
+ * advance by a cost set per grid size, and a device that starts a launch when
+ * it is through with the one before and the host has made it. */
 #include <stddef.h>
 #include <stdlib.h>
 #include <string.h>
@@ -29,10 +32,44 @@ API int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const voi
 }
 API int cudaStreamCreateWithFlags(void** s, unsigned f) { return (void)f, *s = malloc(1), kOk; }
 API int cudaStreamDestroy(void* s) { return free(s), kOk; }
-API int cudaStreamSynchronize(void* s) { return (void)s, fail_sync ? kUnknown : kOk; }
-API int cudaEventCreate(void** e) { return *e = malloc(1), kOk; }
-API int cudaEventCreateWithFlags(void** e, unsigned f) { return (void)f, *e = malloc(1), kOk; }
+/* the clocks, in us; a graph is the sum of its kernels' costs */
+static double host_us, device_us, capture_us = -1;
+static double cost_us[1 << 16]; /* by grid size */
+static unsigned lcg;
+static double noise(void) { return lcg = lcg * 1664525u + 1013904223u, (lcg >> 8) / 16777216.0; }
+static void run(double us) {
+  if (capture_us >= 0) capture_us += us;
+  else device_us = (device_us > host_us ? device_us : host_us) + us;
+}
+static void* boxed(double v) { return memcpy(malloc(sizeof v), &v, sizeof v); }
+
+API void fake_cost(int grid, double us) { cost_us[grid] = us; }
+API void fake_seed(unsigned s) { lcg = s; }
+
+API int cudaStreamSynchronize(void* s) {
+  (void)s;
+  if (device_us > host_us) host_us = device_us;
+  return fail_sync ? kUnknown : kOk;
+}
+API int cudaStreamBeginCapture(void* s, int mode) { return (void)s, (void)mode, capture_us = 0, kOk; }
+API int cudaStreamEndCapture(void* s, void** g) { return (void)s, *g = boxed(capture_us), capture_us = -1, kOk; }
+API int cudaGraphInstantiate(void** e, void* g, unsigned long long f) {
+  return (void)f, host_us += 1000, *e = boxed(*(double*)g), kOk;
+}
+API int cudaGraphDestroy(void* g) { return free(g), kOk; }
+API int cudaGraphExecDestroy(void* e) { return free(e), kOk; }
+/* a launch takes the host 4 to 12 us */
+API int cudaGraphLaunch(void* e, void* s) { return (void)s, host_us += 4 + 8 * noise(), run(*(double*)e), kOk; }
+API int cudaEventCreate(void** e) { return *e = boxed(0), kOk; }
+API int cudaEventCreateWithFlags(void** e, unsigned f) { return (void)f, *e = boxed(0), kOk; }
 API int cudaEventDestroy(void* e) { return free(e), kOk; }
+API int cudaEventRecord(void* e, void* s) {
+  return (void)s, host_us += 1, *(double*)e = device_us > host_us ? device_us : host_us, kOk;
+}
+API int cudaEventSynchronize(void* e) { return host_us = host_us > *(double*)e ? host_us : *(double*)e, kOk; }
+API int cudaEventElapsedTime(float* ms, void* a, void* b) {
+  return *ms = (float)((*(double*)b - *(double*)a) * 1e-3), kOk;
+}
 API int cudaMalloc(void** p, size_t n) { return *p = calloc(n ? n : 1, 1), *p ? kOk : 2; }
 API int cudaFree(void* p) { return free(p), kOk; }
 API int cudaMemset(void* p, int v, size_t n) { return memset(p, v, n), kOk; }
@@ -54,4 +91,7 @@ API int cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w
   return rc;
 }
 API int cudaLaunchKernel(const void* f, ...) { return (void)f, kOk; }
-API int cudaLaunchKernelExC(const void* c, const void* f, void** a) { return (void)c, (void)f, (void)a, kOk; }
+API int cudaLaunchKernelExC(const void* c, const void* f, void** a) {
+  const unsigned grid = *(const unsigned*)c; /* the configuration begins with gridDim.x */
+  return (void)f, (void)a, run(grid < 1 << 16 ? cost_us[grid] : 0), kOk;
+}

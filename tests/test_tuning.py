@@ -1,0 +1,32 @@
+"""The choice of the sweep form: candidates a few percent apart must be told
+apart whatever the host takes to launch a graph.  The CUDA runtime is the model
+of fake_cudart.c (a launch costs the host 4 to 12 us), so the fastest form is
+known and the test runs without a GPU."""
+import pytest
+
+from test_reads import fake  # noqa: F401
+
+# FP64 16^3 (2048 sites per parity): 16 tiles of 128 sites, 8 of 256, 4 of 2 x 256
+TILES = {(128, 1): 16, (256, 1): 8, (256, 2): 4}
+
+
+@pytest.mark.parametrize("calls", [[60], [16] + [5] * 10, [3] * 20, [4] * 16])
+@pytest.mark.parametrize("fastest", sorted(TILES))
+def test_the_fastest_form_is_chosen(fake, fastest, calls):  # noqa: F811
+    """Ten passes of 7.5 us or 7.65 us: 75 against 76.5 us per sweep."""
+    fake(f"""
+for shape, tiles in {TILES!r}.items():
+    fake.fake_cost(tiles, C.c_double(7.5 if shape == {fastest!r} else 7.65))
+threads, spt, regs, wrong = C.c_int(), C.c_int(), C.c_int(), 0
+for seed in range(20):
+    fake.fake_seed(seed * 7919 + 1)
+    p = (_lib.LceParams * 1)(Params(L=(16, 16, 16), precision="f64", seed=1).to_c())
+    c = lib.lce_create_batch(p, 1)
+    for n in {calls!r}:
+        assert lib.lce_sweeps(c, n, 0) == 0
+    assert lib.lce_get_sweep_mode(c) in (_lib.LCE_SWEEP_PASSES, _lib.LCE_SWEEP_PASSES2)
+    lib.lce_get_tile_shape(c, C.byref(threads), C.byref(spt), C.byref(regs))
+    wrong += (threads.value, spt.value) != {fastest!r}
+    lib.lce_destroy(c)
+assert wrong == 0, f"{{wrong}} of 20 contexts chose a slower form"
+""")
