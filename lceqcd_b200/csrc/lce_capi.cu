@@ -581,7 +581,8 @@ int enqueue_persistent(lce_ctx* c, const std::vector<unsigned char>& routines, i
   return LCE_OK;
 }
 
-constexpr int kTuneSweeps = 4;
+constexpr int kTuneSweeps = 3;
+constexpr long kTuneRunSites = 1L << 20;
 
 // Graphs of several sweeps defer each sweep's finalize (but the last) into an
 // extra block of the next sweep's first pass (higgs_fin_kernel): a single
@@ -678,17 +679,19 @@ std::vector<unsigned char> sweep_routines(const lce_ctx* c) {
 }
 
 // Autotune on real sweeps: each candidate (sweep form and tile shape) runs one
-// discarded sweep and kTuneSweeps timed ones, and the fastest is kept.  The
-// timed sweeps of a candidate are replayed back to back between two events, the
-// candidates' runs queued behind one another.  Events around a single sweep, with
-// a synchronisation after each, also timed the host's launch of its graph (8 us,
-// +- 1.5 us), and events on a busy stream come in steps of 2.05 us, so in either
-// way shapes a few percent apart were taken for one another.  Of 24 fresh
-// contexts the faster shape now goes to 20 at 32^3 in FP32 (28.6 against 30.8 us
-// per sweep; 10 with the median of three single sweeps), to 24 at 24^3 (27.0,
-// 28.4; 21), and in FP64 to 24 at 56^3 (70.9, 72.2; 23) as at 48^3 and 64^3.  A
-// call's first sweep, behind an idle stream, is not timed unless every sweep is a
-// call of its own.  Adds the sweeps queued to *done.
+// discarded sweep and kTuneSweeps timed ones, and the fastest by median is kept.
+// The sweeps of a call are queued behind one another with events between them:
+// with a synchronisation after each, a sample also held the host's launch of the
+// graph (8 us, +- 1.5 us).  Up to kTuneRunSites sites (a sweep of ~0.2 ms) a
+// candidate's timed sweeps run back to back between two events, because events
+// on a busy stream come in steps of 2.05 us; either error took shapes a few
+// percent apart for one another (the faster of two at 32^3 FP32, 28.6 against
+// 30.8 us per sweep, in 14 of 18 fresh contexts; 9 with the median of three
+// single sweeps).  Larger lattices take one sweep of each
+// candidate in turn: their sweeps draw the power that slows the clocks while the
+// tuning runs (256^3: a run of four of the first candidates came out 4% faster
+// than they are).  A call's first sweep, behind an idle stream, is not part of a
+// run.  Adds the sweeps queued to *done.
 int tune_sweeps(lce_ctx* c, int nsweeps, int mf, int* done) {
   struct Run {
     int form, sweeps;  // form -1: not timed
@@ -696,10 +699,13 @@ int tune_sweeps(lce_ctx* c, int nsweeps, int mf, int* done) {
   std::vector<Run> runs;
   std::vector<int> had;  // each candidate's sweeps, the discarded one included
   for (const TuneForm& f : c->tune) had.push_back(f.sweeps);
+  long sites = 0;
+  for (const ChainDev& d : c->ch) sites += 2L * d.nh;
+  const bool by_runs = nsweeps > 1 && sites <= kTuneRunSites;
   while (*done < nsweeps) {
-    auto next = std::find(had.begin(), had.end(), 0);
-    if (next == had.end()) next = std::find_if(had.begin(), had.end(), [](int n) { return n <= kTuneSweeps; });
-    if (next == had.end()) break;
+    auto next = std::min_element(had.begin(), had.end());
+    if (*next > kTuneSweeps) break;
+    if (by_runs && *next > 0) next = std::find_if(had.begin(), had.end(), [](int n) { return n <= kTuneSweeps; });
     const int k = (int)(next - had.begin()), left = nsweeps - *done;
     const TuneForm tf = c->tune[k];
     cudaGraphExec_t ex = nullptr;
@@ -712,8 +718,8 @@ int tune_sweeps(lce_ctx* c, int nsweeps, int mf, int* done) {
       CK(cudaEventCreate(&e));
       c->tune_ev.push_back(e);
     }
-    const bool idle = *next > 0 && runs.empty() && left > 1;
-    const int m = *next == 0 || idle ? 1 : std::min(left, 1 + kTuneSweeps - *next);
+    const bool idle = by_runs && *next > 0 && runs.empty() && left > 1;
+    const int m = by_runs && *next > 0 && !idle ? std::min(left, 1 + kTuneSweeps - *next) : 1;
     if (runs.empty()) CK(cudaEventRecord(c->tune_ev[0], c->stream));
     for (int i = 0; i < m; ++i) {
       if (ex) CK(cudaGraphLaunch(ex, c->stream));

@@ -37,14 +37,20 @@ static double host_us, device_us, capture_us = -1;
 static double cost_us[1 << 16]; /* by grid size */
 static unsigned lcg;
 static double noise(void) { return lcg = lcg * 1664525u + 1013904223u, (lcg >> 8) / 16777216.0; }
+static double slowing, busy_us; /* the device slows by this share per us of work it has done */
 static void run(double us) {
-  if (capture_us >= 0) capture_us += us;
-  else device_us = (device_us > host_us ? device_us : host_us) + us;
+  if (capture_us >= 0) {
+    capture_us += us;
+    return;
+  }
+  device_us = (device_us > host_us ? device_us : host_us) + us * (1 + slowing * busy_us);
+  busy_us += us;
 }
 static void* boxed(double v) { return memcpy(malloc(sizeof v), &v, sizeof v); }
 
 API void fake_cost(int grid, double us) { cost_us[grid] = us; }
 API void fake_seed(unsigned s) { lcg = s; }
+API void fake_slowing(double per_us) { slowing = per_us, busy_us = 0; }
 
 API int cudaStreamSynchronize(void* s) {
   (void)s;
