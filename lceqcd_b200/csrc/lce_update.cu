@@ -787,14 +787,15 @@ __device__ __forceinline__ void finalize_small_body(const FinalizeArgs& f, Small
   if (!DEFERRED) pdl_wait();
   const int nch = f.nchunks, b1 = f.ntiles0;  // chain 0's chunks and tiles, from the host
   // chunk sums summed behind: one chunk -> the total, else chunks[k][i]
-  // (the slots [0, pre) of one chunk are pre * kNQ consecutive doubles)
-  if ((int)threadIdx.x < f.pre * kNQ) {
-    const int i = threadIdx.x / kNQ, q = threadIdx.x % kNQ;
+  // (the slots [0, pre) of one chunk are pre * kNQ consecutive doubles, up to
+  // 252: more than a block of 128 threads takes in one step)
+  for (int e = threadIdx.x; e < f.pre * kNQ; e += blockDim.x) {
+    const int i = e / kNQ, q = e % kNQ;
 #pragma unroll
     for (int k = 0; k < kSmallChunks; ++k) {
       if (k < nch)
         S.ck[(i * kSmallChunks + k) * kNQ + q] =
-            nch == 1 ? __ldcg(f.totals + threadIdx.x) : __ldcg(f.chunks + (size_t)k * kMaxSlots * kNQ + threadIdx.x);
+            nch == 1 ? __ldcg(f.totals + e) : __ldcg(f.chunks + (size_t)k * kMaxSlots * kNQ + e);
     }
   }
   // level 1 of the remaining slots
