@@ -367,7 +367,10 @@ __device__ __forceinline__ void link_tile(const Args<ONE>& p, int tile) {
     Uniforms<R, OR ? 1 : 7> Un = Un0;
     if (r == 0 && early ? ok0 : setup_uniforms<R, OR ? 1 : 7>(p, ch, s, OR ? kPlanar : kTriple, Un)) {
       const su2<R> V = staple<R, MU, PDL, ONE>(ch, eo, no, s);
-      su2<R> uo = ldU<R, PDL, ONE>(ch, MU, eo, s);
+      // (kTable: the index formed once and kept for the store; formed again
+      // there, the FP64 persistent sweep of 12^3 took 70.6 us instead of 69.0)
+      const size_t li = (size_t)(MU * 2 + eo) * nh + s;
+      su2<R> uo = ONE ? ldU<R, PDL, ONE>(ch, MU, eo, s) : (PDL ? LinkIO<R>::ld(ch.u, li) : LinkIO<R>::ld_cg(ch.u, li));
       // f/agauge.f:71-84: normalised staple, 1/(beta |V|), 1/2 Re Tr(U Vhat)
       const R tn = M<R>::rsqrt(norm2(V));
       const su2<R> vh{{tn * V.a.re, tn * V.a.im}, {tn * V.b.re, tn * V.b.im}};
@@ -422,7 +425,7 @@ __device__ __forceinline__ void link_tile(const Args<ONE>& p, int tile) {
       if (changed) {
         const su2<R> un = p.fuse_renorm ? unitarise64(uo) : uo;
         if (ONE) LinkIO<R>::st(static_cast<char*>(ch.u) + (size_t)(MU * 2 + eo) * nh * LinkIO<R>::kBytes, s, un);
-        else LinkIO<R>::st(ch.u, (size_t)(MU * 2 + eo) * nh + s, un);
+        else LinkIO<R>::st(ch.u, li, un);
       }
       // f/agauge.f:179-185 plaquette against the staple
       if (!OR && p.part) pl[0] += (double)nn(uo, V).a.re;
