@@ -237,6 +237,7 @@ bool valid_params(const lce_params& p, std::string& why) {
 // creation, and the copy is a few hundred bytes.
 constexpr size_t kReportState = 256;
 static_assert(sizeof(CtxState) <= kReportState, "the measurements follow the state");
+static_assert(sizeof(CtxState) <= sizeof(lce_meas), "one row of lce_get_meas holds either");
 size_t report_bytes(int nrec) { return kReportState + sizeof(lce_meas) * nrec; }
 lce_meas* report_meas(lce_ctx* c) {
   return reinterpret_cast<lce_meas*>(reinterpret_cast<char*>(c->report.data()) + kReportState);
@@ -2321,10 +2322,14 @@ int lce_sweep(lce_ctx* c, int measflag, lce_meas* m) {
 int lce_get_meas(lce_ctx* c, int chain, lce_meas* m) {
   DeviceScope ds_(c ? c->device : -1);
   if (!c || !m || chain < 0 || chain >= c->nchains) return LCE_ERR_INVALID;
-  // chain 0's record follows the state; another chain's is a copy of its own
-  if (chain > 0)
-    CK(cudaMemcpyAsync(report_meas(c) + chain, c->meas_d + chain, sizeof(*m), cudaMemcpyDeviceToHost, c->stream));
-  if (const int rc = report_read(c, chain > 0 ? 0 : 1)) return rc;
+  if (chain == 0) {
+    if (const int rc = report_read(c, 1)) return rc;
+  } else {
+    // the state and a later chain's record as the two rows of one copy
+    const size_t pitch = report_bytes(chain);
+    CK(cudaMemcpy2DAsync(c->report.data(), pitch, c->st_d, pitch, sizeof(lce_meas), 2, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
   *m = report_meas(c)[chain];
   return report_status(c);
 }
