@@ -1031,8 +1031,8 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
     lce_destroy(c);
     return nullptr;
   }
-  // tile shape: FP32 contexts tune threads per block (128, 256, 512) and sites
-  // per thread under AUTO unless tile_threads fixes the block; FP64 contexts
+  // tile shape: FP32 contexts tune threads per block (128, 256, 448, 512) and
+  // sites per thread under AUTO unless tile_threads fixes the block; FP64 contexts
   // tune 128 or kBlock threads under AUTO if tile_threads leaves it open, and
   // use kBlock otherwise, as z-slabs do
   c->tile_req = !slab && (c->prec == LCE_PREC_F32 || p[0].tile_threads == 0) ? p[0].tile_threads : kBlock;
@@ -1090,13 +1090,12 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
     c->scratch_n = std::max(c->scratch_n, (size_t)21 * d.L3 + 5 + slice_part_doubles(d.nxy, d.L3));
   if ((e = cudaMalloc(&c->scratch_d, sizeof(double) * c->scratch_n)) != cudaSuccess)
     return bail(e, "cudaMalloc(scratch)");
-  if (c->max_L3 * 14 * sizeof(double) > 48 * 1024) {
-    // correlator kernel stages the slice sums in shared memory
-    if (c->max_L3 * 14 * sizeof(double) > 200 * 1024) {
-      g_create_error = "create: L3 too large for the correlator kernel";
-      lce_destroy(c);
-      return nullptr;
-    }
+  // L3 up to 1828: 14 columns of slice sums in 200 KB, the limit as it always
+  // was (correlators_kernel stages at most 12 of them in shared memory)
+  if (c->max_L3 * 14 * sizeof(double) > 200 * 1024) {
+    g_create_error = "create: L3 too large for the correlator kernel";
+    lce_destroy(c);
+    return nullptr;
   }
   return c;
 }

@@ -642,8 +642,6 @@ __global__ void __launch_bounds__(kFaThreads, LOGN <= 8 ? 4 : 1) fa_fft_kernel(F
   }
 }
 
-// (6) inverse FFT along x; g(x) = exp(-i omega.sigma) per site (CG: the
-// direction s = omega + beta s instead)
 // g(x) = exp(-i omega.sigma) of one site into gstep
 __device__ __forceinline__ void fa_site_g(const FaArgs& a, size_t gi, double w3, double wbr, double wbi) {
   const double nw = sqrt(w3 * w3 + wbr * wbr + wbi * wbi);
@@ -663,6 +661,8 @@ __device__ __forceinline__ void fa_site_g(const FaArgs& a, size_t gi, double w3,
   }
 }
 
+// (6) inverse FFT along x; g(x) = exp(-i omega.sigma) per site (CG: the
+// direction s = omega + beta s instead)
 template <typename R, int LOGN, bool CG = false>
 __global__ void __launch_bounds__(kFaThreads) fa_g_kernel(FaArgs a) {
   using G = FaLines<LOGN>;

@@ -195,7 +195,7 @@ struct PassArgsOne : PassArgs {
 // kParamChains chains (22.5 KB of arguments) and at least kParamTiles tiles
 // per pass.  Below that a pass is launch-bound and the larger argument block
 // costs more than it gives (2 chains of 8^3: 29.4 -> 30.6 us per sweep, 12 of
-// 16^3, 192 tiles: 35.0 -> 35.7; 24 of 16^3-32^3, 1584 tiles: 85.3 -> 81.9).
+// 16^3, 192 tiles: 35.0 -> 35.7; 24 of 16^3 and 32^3, 1728 tiles: 93.2 -> 89.0).
 constexpr int kParamChains = 128, kParamTiles = 512;
 struct PassArgsMany : PassArgs {
   int many;

@@ -557,11 +557,14 @@ constexpr int min_blocks_bs() {
 // without measurements, the same tile: 16^3 22.1 -> 20.4 us, 64^3 38.6 ->
 // 36.6, with 4 overrelaxations 125.0 -> 115.8, 128^3 301 -> 290, FP64 64^3
 // 93.8 -> 88.8.  kMany: a batch's table in the parameter bank, found by the
-// block's tile: 96 chains of 16^3-48^3 with two sites per thread 796 -> 762
-// us, one 836 -> 818.  kTable: the table in memory (kParamTiles).  The passes
-// of 64^3 and above are bound by instruction issue (a link heatbath takes
-// ~700 warp instructions per site, 335 of them FP32 arithmetic, ~70% of the
-// issue slots of an active SM).
+// block's tile: 96 chains of 16^3-48^3 with two sites of 128 threads 829 -> 802
+// us per measured sweep, one site 880 -> 817; 64 of 32^3 382 -> 366 and 402 ->
+// 370, in FP64 772 -> 718.  kTable: the table in memory (kParamTiles).  The FP32
+// passes of 64^3 and above are bound by instruction issue: at 128^3 a link
+// heatbath takes 775 warp instructions per site, 309 of them FP32 adds,
+// multiplies and multiply-adds, and 68% of the issue slots of an active SM.  The
+// FP64 ones are not (64^3: issue 37%, FP64 pipe 28%): their 80 registers leave
+// 18 warps per SM to hide the latency of the loads.
 template <typename R, int MODE, int SPT, int BS, int OCC, int ONE>
 __global__ void __launch_bounds__(BS, min_blocks_bs<R, BS, OCC>()) higgs_kernel(Args<ONE> p) {
   if (kReduceBehind<SPT> && p.rb_nitems && (int)blockIdx.x >= p.ntiles) reduce_behind(p);
@@ -1098,10 +1101,12 @@ void launch_link_t(int mode, int mu, const PassArgsMany& a, int nblocks, cudaStr
 // {128, 256} x {2} at the 64-register cap, (448, 1) at two blocks per SM (72
 // registers), and (128, 1) at 56 registers (a.occ = 1152); FP64 (256, 1),
 // (256, 2) and (128, 1).  FP64 with 128 instead of 256 threads, us per sweep
-// with measurements: 8^3 36.1 -> 32.6 and 24^3 41.0 -> 38.2 (few blocks: a
-// pass is the latency of the SM with the most warps), 32^3 41.6 -> 41.5, 48^3
-// 63.8 -> 66.1, 64^3 96.6 -> 94.6 (a finer last wave); a looser register cap
-// (128) changed nothing.  The autotuner tells them apart.
+// with measurements, in graphs of 8 sweeps and of one: 8^3 38.6 -> 35.2, 24^3
+// 42.1 -> 38.7 and 47.2 -> 43.1 (few blocks: a pass is the latency of the SM
+// with the most warps), 32^3 41.3 -> 42.0 and 47.2 -> 45.1, 40^3 51.6 -> 50.1
+// and 51.3 -> 49.4, 48^3 63.8 -> 65.8 and 59.4 -> 55.4, 56^3 70.9 -> 72.2 (8),
+// 64^3 96.5 -> 94.3 and 102.5 -> 98.6 (a finer last wave); a looser register cap
+// (128) changed nothing.  The autotuner tells them apart, by graphs of one.
 template <typename R>
 void launch_higgs(int mode, const PassArgsMany& a, int nblocks, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
