@@ -247,7 +247,8 @@ int lce_get_sweep_mode(lce_ctx* ctx);
  * thread and the per-thread register cap they are compiled for (a tuned
  * choice once lce_get_sweep_mode is no longer AUTO); any output may be NULL */
 int lce_get_tile_shape(lce_ctx* ctx, int* threads, int* sites_per_thread, int* register_cap);
-/* f/meas1.f inputs: the last measured quantities of a chain */
+/* f/meas1.f inputs: the last measured quantities of a chain (of every chain);
+ * m is written unless the read itself fails (LCE_ERR_CUDA from the copy) */
 int lce_get_meas(lce_ctx* ctx, int chain, lce_meas* m);
 int lce_get_meas_batch(lce_ctx* ctx, lce_meas* m /* [nchains] */);
 
