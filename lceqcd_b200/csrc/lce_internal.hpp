@@ -98,7 +98,7 @@ struct CtxState {
   unsigned long long stream_pos;  // validation-stream position
   unsigned int status;            // LCE_STATUS_* bits
   unsigned int ticket;            // last-block ticket of the finalize kernel
-  // the buffers of the reduce-behind blocks (lce_update.cu), set at context
+  // the buffers of the reduce-behind blocks (lce_passes.cuh), set at context
   // creation: tile partials (slot i at rb_part + i * rb_slot_stride), the
   // chunk table of each tile table, chunk sums and totals
   const double* rb_part;
@@ -175,7 +175,7 @@ struct PassArgs {
   int rng_early;
   // reduce-behind: blocks [ntiles, gridDim.x) of a per-pass launch sum the
   // previous pass's tile partials (slot rb_slot & 0xff, tile table rb_slot >>
-  // 8; the buffers in *st) into level-1 chunk sums (lce_update.cu), the same
+  // 8; the buffers in *st) into level-1 chunk sums (lce_passes.cuh), the same
   // additions in the same order as the finalize kernel's level 1, while this
   // pass's tiles update sites; rb_nitems = 0: no previous slot.  (Three ints
   // here: a larger argument block changed the register allocation of the
@@ -183,7 +183,7 @@ struct PassArgs {
   int ntiles, rb_slot, rb_nitems;
 };
 // with a single-chain context's chain, for the kernels that read it from the
-// parameter bank (lce_update.cu: ONE)
+// parameter bank (lce_passes.cuh: ONE)
 struct PassArgsOne : PassArgs {
   ChainDev one;
   // its couplings in FP32 (FP32 contexts)
@@ -217,7 +217,7 @@ struct FinalizeArgs {
   unsigned int npasses;           // advance of st->pass_ctr
   unsigned long long nstream;     // advance of st->stream_pos
   int single;                     // FP32 arithmetic for the ahiggs1 step update
-  // two-level reduction of the tile partials (lce_update.cu): chunks of 128
+  // two-level reduction of the tile partials (lce_passes.cuh): chunks of 128
   // tiles; chunk_begin = nchains + 1 prefix of chunks per chain
   const int* chunk_begin;
   double* chunks;                 // [chunk][kMaxSlots][kNQ]
