@@ -426,10 +426,13 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* part, 
 // iteration's check is made by the next one's first half-step (gf_prev_stops).
 // 128 threads up to 8192 sites per parity, where blocks of 256 leave most of
 // the chip idle (16^3 6.97 -> 6.52 us per iteration, FP64 6.67 -> 5.45; at 48 x
-// 40 x 36 256 is better, 12.00 against 12.27).  Up to 1024 partials every block
-// can add them (64^3, 512 of them: an iteration 14.7 -> 12.9 us, 8^3 8.6 ->
-// 6.2); at 128^3, 4096, the check kernel's 4 of 82 us are the cheaper.
-constexpr int kGfSmallBlock = 128, kGfSmallSites = 8192, kGfMaxPartials = 1024;
+// 40 x 36 256 is better, 12.00 against 12.27).  Up to 512 partials every block
+// can add them (us per iteration with a check kernel against the fold: 16^3
+// 8.0 / 6.8, FP64 9.3 / 8.1; 48 x 40 x 36 9.3 / 7.6, FP64 12.5 / 11.2; 64^3, 512
+// of them, 14.1 / 13.2, FP64 27.6 / 27.8).  Beyond that the blocks' adds cost more
+// than the kernel: 64 x 64 x 80, 640 partials, 16.9 / 16.7 and in FP64 31.6 /
+// 33.8, 64 x 64 x 116, 928, 20.2 / 20.6 and 39.5 / 43.7.
+constexpr int kGfSmallBlock = 128, kGfSmallSites = 8192, kGfMaxPartials = 512;
 int gf_block(int nh) { return nh <= kGfSmallSites ? kGfSmallBlock : kBlock; }
 int gf_folds(int nh) {
   const int nb = ceil_div(nh, gf_block(nh));

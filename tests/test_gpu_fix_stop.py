@@ -1,6 +1,6 @@
 """The iteration at which a gauge fixing stops: the first one whose theta is at
 or below the limit, whether the check is made by the next iteration's first
-half-step (up to 1024 theta partials) or by a kernel of its own, and wherever
+half-step (up to 512 theta partials) or by a kernel of its own, and wherever
 in a batch of 8, 16, ... iterations that iteration lies."""
 import ctypes as C
 
@@ -40,8 +40,8 @@ def configuration(L):
     return u, a
 
 
-# sites per parity: 480; 8448 (blocks of 256); 262144 (1024 partials); 266240 (1040: a check kernel)
-@pytest.mark.parametrize("L", [(12, 10, 8), (32, 44, 12), (64, 64, 128), (64, 64, 130)])
+# sites per parity: 480; 8448 (blocks of 256); 131072 (512 partials); 135168 (528: a check kernel); 262144; 266240
+@pytest.mark.parametrize("L", [(12, 10, 8), (32, 44, 12), (64, 64, 64), (64, 64, 66), (64, 64, 128), (64, 64, 130)])
 @pytest.mark.parametrize("form", ["plain", "tracked", "iterative"])
 def test_stops_at_the_first_theta_within_the_limit(L, form):
     u, a = configuration(L)
