@@ -1083,7 +1083,7 @@ lce_ctx* create_impl(const lce_params* p, int n, const SlabInfo* slab = nullptr)
       return bail(e, "cudaMemcpy(state)");
   }
   c->scratch_n = (size_t)2 * ceil_div(2L * c->max_nh, 256) + (size_t)32 * c->max_L3 + 64;
-  // gauge fixing: at most 1024 theta partials of small blocks
+  // gauge fixing: the theta partials (64 of small blocks, 512 folded into the check)
   c->scratch_n = std::max(c->scratch_n, (size_t)1024);
   // slice measurements: sums, output and the segments' partial sums
   for (const ChainDev& d : c->ch)
